@@ -36,7 +36,7 @@ void block_faces(const int ex[3], const double* X, const double* Y, const double
 template <typename T, typename SS, bool SYMM, bool SPLIT, bool Z4C>
 cudaError_t launch_substep(const void* blocks, const int2* tiles, int ntiles, int sub, RKConst rk, int enforce,
                            unsigned* status, int grid, cudaStream_t s, const void* D, long long dfs);
-template <typename T, typename SS, bool SYMM>
+template <typename T, typename SS>
 cudaError_t launch_face(const void* blocks, const int2* faces, int nfaces, int sub, RKConst rk, int enforce,
                         unsigned* status, cudaStream_t s);
 template <typename T, typename SS>
@@ -156,7 +156,7 @@ int fwd_step(amss_adjoint* a, const double* U0raw, double* Unew, double* Z0, dou
     AMSS_CK((launch_deriv<double, double>(T, a->ditems, a->nitems, sub, D, a->fs, std::min(a->nitems, 148 * 16), s, 0)));
     AMSS_CK((launch_substep<double, double, false, true, false>(T, a->dtiles, a->ntiles, sub, rk, 0, a->dstatus,
                                                               std::min(a->ntiles, 148 * 8), s, D, a->fs)));
-    AMSS_CK((launch_face<double, double, false>(T, a->dfaces, a->nfaces, sub, rk, 0, a->dstatus, s)));
+    AMSS_CK((launch_face<double, double>(T, a->dfaces, a->nfaces, sub, rk, 0, a->dstatus, s)));
     a->launches += 3;
     if (sub < 3) {
       k_enforce_copy<<<grid_of(n), 128, 0, s>>>(Z[sub], a->X[sub], n, fs);
@@ -261,7 +261,6 @@ extern "C" amss_adjoint* amss_adjoint_create(const int ex[3], const double bbox[
   block_faces(ex, xs[0], xs[1], xs[2], bbox, 0, &s.b.face_mask, &s.b.lowsym_mask);
   s.C.t = make_coef<double>(s.b.dx, eps);
   s.C.d = s.C.t;
-  for (int d = 0; d < 3; ++d) s.d2s[d] = 1.0 / 2.0 / a->dx[d];
   s.lvl = a->dlvl;
   s.doff = 0;
   s.npts = a->npts;
@@ -271,7 +270,7 @@ extern "C" amss_adjoint* amss_adjoint_create(const int ex[3], const double bbox[
   for (int t = 0; t < 4; ++t) a->host_tab[t] = s;
   a->host_adj.b = s.b;
   a->host_adj.C = s.C;
-  for (int d = 0; d < 3; ++d) a->host_adj.d2s[d] = s.d2s[d];
+  for (int d = 0; d < 3; ++d) a->host_adj.d2s[d] = s.C.d.d2[d];
   a->host_adj.npts = a->npts;
   a->host_adj.D = a->D;
   a->host_adj.dfs = a->fs;

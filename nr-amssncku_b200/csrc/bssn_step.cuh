@@ -76,7 +76,6 @@ struct EpiRK {
   double* out_side;   // FP64 side slots (chi, alpha, beta^i) of an FP32 stage output
   long long fs, p;
   int sub;
-  bool freeze;        // outer face of a refined patch: output = u0 there
   bool enforce;
   RKConst c;
   double g[6], a[6];
@@ -87,10 +86,7 @@ struct EpiRK {
     const double k = (double)kv;
     const double u = u0[o];
     double r;
-    if (freeze) {
-      // a frozen point's accumulator is never read (it would only feed r)
-      r = u;
-    } else if (sub == 0) {
+    if (sub == 0) {
       r = u + c.half_dt * k;
       K[o] = k;
     } else if (sub == 1) {
@@ -129,44 +125,11 @@ struct EpiRK {
   }
 };
 
-// Sommerfeld RHS of one field at an outer-face point
-// (sommerfeld_rout.f90:378-440, "new code, 2012dec26"):
-//   rhs = -v (x fx + y fy + z fz + f) / r, one-sided 2nd order, upwinded by
-//   the sign of v x_d / r.  imin/imax are 0-based; lo = -1 at a symmetry plane.
-template <typename T, int F, typename P>
-__device__ __forceinline__ T sommerfeld_point(const P& q, const T (&d2)[3], const int (&lo)[3], const int (&hi)[3],
-                                             T x, T y, T z, T velocity) {
-  const T R = sqrt(x * x + y * y + z * z);
-  const T w[3] = {velocity * x / R, velocity * y / R, velocity * z / R};
-  const int id[3] = {q.i, q.j, q.k};
-  T fd[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    auto f = [&](int o) -> T {
-      return q.template vpad<T, F>(d == 0 ? o : 0, d == 1 ? o : 0, d == 2 ? o : 0);
-    };
-    T r = T(0);
-    if (w[d] > T(0)) {
-      if (id[d] - 2 >= lo[d]) r = d2[d] * (T(3) * f(0) - T(4) * f(-1) + f(-2));
-      else if (id[d] - 1 >= lo[d]) r = d2[d] * (-f(-1) + f(1));
-      else r = d2[d] * (-f(2) + T(4) * f(1) - T(3) * f(0));
-    } else if (w[d] < T(0)) {
-      if (id[d] + 2 <= hi[d]) r = d2[d] * (-f(2) + T(4) * f(1) - T(3) * f(0));
-      else if (id[d] + 1 <= hi[d]) r = d2[d] * (-f(-1) + f(1));
-      else r = d2[d] * (T(3) * f(0) - T(4) * f(-1) + f(-2));
-    }
-    fd[d] = r;
-  }
-  const T f0 = q.template v<T, F>(0, 0, 0);
-  return -velocity * (fd[0] * x + fd[1] * y + fd[2] * z + f0) / R;
-}
-
 // One block of a level as the fused substep sees it.
 template <typename T>
 struct StepBlock {
   BlockView b;
   Coefs<T> C;
-  T d2s[3];           // 1/2/dx for the Sommerfeld rule
   double* tl[3];      // three time levels of the FP64 state: tl[cur] = U0 (t_n),
                       // tl[(cur+1)%3] receives U_new (it held t_n - 2 dt)
   const int* lvl;     // level state {cur, steps taken} (device, rotated after each step)

@@ -33,7 +33,7 @@ void block_faces(const int ex[3], const double* X, const double* Y, const double
 template <typename T, typename SS, bool SYMM, bool SPLIT, bool Z4C>
 cudaError_t launch_substep(const void* blocks, const int2* tiles, int ntiles, int sub, RKConst rk, int enforce,
                            unsigned* status, int grid, cudaStream_t s, const void* D, long long dfs);
-template <typename T, typename SS, bool SYMM>
+template <typename T, typename SS>
 cudaError_t launch_face(const void* blocks, const int2* faces, int nfaces, int sub, RKConst rk, int enforce,
                         unsigned* status, cudaStream_t s);
 template <typename T, typename SS>
@@ -345,7 +345,6 @@ static int build_table(amss_engine* e, ELevel& L, int level) {
     s.b.lowsym_mask = b.lowsym;
     s.C.t = make_coef<T>(s.b.dx, e->prm.eps);
     s.C.d = make_coef<double>(s.b.dx, e->prm.eps);
-    for (int d = 0; d < 3; ++d) s.d2s[d] = (T)(1.0 / 2.0 / s.b.dx[d]);
     for (int t = 0; t < 3; ++t) s.tl[t] = b.tl[t];
     s.lvl = e->dlvl + 2 * level;
     s.stage[0] = b.st[0];
@@ -828,10 +827,8 @@ static int step_level_impl(amss_engine* e, int level, double dt, bool fin = fals
     // regions, past which the faces lie.
     auto face = [&](int s) -> cudaError_t {
       e->launches++;
-      return mixed ? (L.symm ? launch_face<float, float, true>(L.dtable, L.dfaces, L.nfaces, s, rk, enf, e->dstatus, e->stream)
-                             : launch_face<float, float, false>(L.dtable, L.dfaces, L.nfaces, s, rk, enf, e->dstatus, e->stream))
-                   : (L.symm ? launch_face<double, double, true>(L.dtable, L.dfaces, L.nfaces, s, rk, enf, e->dstatus, e->stream)
-                             : launch_face<double, double, false>(L.dtable, L.dfaces, L.nfaces, s, rk, enf, e->dstatus, e->stream));
+      return mixed ? launch_face<float, float>(L.dtable, L.dfaces, L.nfaces, s, rk, enf, e->dstatus, e->stream)
+                   : launch_face<double, double>(L.dtable, L.dfaces, L.nfaces, s, rk, enf, e->dstatus, e->stream);
     };
     if (L.nfaces) {
       if (level == 0) {

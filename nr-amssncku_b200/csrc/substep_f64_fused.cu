@@ -5,6 +5,4 @@
 namespace amss {
 template cudaError_t launch_substep<double, double, false, false, false>(const void*, const int2*, int, int, RKConst, int,
                                                        unsigned*, int, cudaStream_t, const void*, long long);
-template cudaError_t launch_face<double, double, false>(const void*, const int2*, int, int, RKConst, int, unsigned*,
-                                                cudaStream_t);
 }  // namespace amss

@@ -117,7 +117,6 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? AMSS_SUBSTEP_MINB_F32 : 
     epi.sub = sub;
     epi.enforce = enforce != 0;
     epi.c = rk;
-    epi.freeze = false;
     const int fm = B.b.face_mask;
     const bool on_face = ((fm & 1) && q.i == q.ex0 - 1) || ((fm & 2) && q.j == q.ex1 - 1) ||
                          ((fm & 4) && q.k == q.ex2 - 1) || ((fm & 8) && q.i == 0) || ((fm & 16) && q.j == 0) ||
@@ -139,50 +138,6 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? AMSS_SUBSTEP_MINB_F32 : 
     }
     if (st) atomicOr(status, st);
   }
-}
-
-// Outer-face points of a level (Sommerfeld on level 0, frozen on refined patch
-// faces), one thread each, from the list faces[] = (block, point).
-template <typename T, typename SI, typename SO, bool SYMM>
-__global__ void __launch_bounds__(128) k_face(const StepBlock<T>* __restrict__ blocks, const int2* __restrict__ faces,
-                                              int nfaces, int sub, RKConst rk, int enforce, unsigned* status) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nfaces; t += gridDim.x * blockDim.x) {
-    const int2 fc = faces[t];
-    const StepBlock<T>& B = blocks[fc.x];
-    const long long p = fc.y;
-    const int cur = B.lvl[0];
-    double* u0 = B.tl[cur];
-    const SI* in = sub == 0 ? (const SI*)u0 : (const SI*)B.stage[sub == 2 ? 1 : 0];
-    auto q = make_pt<SI, SYMM>(in, B.b, p, sub == 0 ? nullptr : B.side[sub == 2 ? 1 : 0]);
-    EpiRK<T, SO> epi;
-    epi.out_side = sub == 3 ? nullptr : B.side[sub == 1 ? 1 : 0];
-    epi.u0 = u0;
-    epi.K = B.K;
-    epi.out = sub == 3 ? (SO*)B.tl[(cur + 1) % 3] : (SO*)B.stage[sub == 1 ? 1 : 0];
-    epi.fs = B.b.fs;
-    epi.p = p;
-    epi.sub = sub;
-    epi.enforce = enforce != 0;
-    epi.c = rk;
-    epi.freeze = false;
-    const unsigned st = face_point<T, SI, SO, SYMM>(B, q, epi);
-    if (st) atomicOr(status, st);
-  }
-}
-
-template <typename T, typename SS, bool SYMM>
-cudaError_t launch_face(const void* blocks, const int2* faces, int nfaces, int sub, RKConst rk, int enforce,
-                        unsigned* status, cudaStream_t s) {
-  if (nfaces == 0) return cudaSuccess;
-  const StepBlock<T>* bl = (const StepBlock<T>*)blocks;
-  const int grid = (nfaces + 127) / 128 < 148 * 8 ? (nfaces + 127) / 128 : 148 * 8;
-  if (sub == 0)
-    k_face<T, double, SS, SYMM><<<grid, 128, 0, s>>>(bl, faces, nfaces, sub, rk, enforce, status);
-  else if (sub == 3)
-    k_face<T, SS, double, SYMM><<<grid, 128, 0, s>>>(bl, faces, nfaces, sub, rk, enforce, status);
-  else
-    k_face<T, SS, SS, SYMM><<<grid, 128, 0, s>>>(bl, faces, nfaces, sub, rk, enforce, status);
-  return cudaGetLastError();
 }
 
 // SPLIT: the pointwise pass of the split form (per-thread loads over
