@@ -33,15 +33,15 @@ template <typename T>
 Coef<T> make_coef(const double dx[3], double eps);
 void block_faces(const int ex[3], const double* X, const double* Y, const double* Z, const double bbox[6],
                  int symmetry, int* face_mask, int* lowsym_mask);
-template <typename T, typename SS, bool SYMM, bool SPLIT, bool Z4C>
-cudaError_t launch_substep(const void* blocks, const int2* tiles, int ntiles, int sub, RKConst rk, int enforce,
-                           unsigned* status, int grid, cudaStream_t s, const void* D, long long dfs);
+template <typename T, typename SS, bool Z4C>
+cudaError_t launch_pointwise(const void* blocks, const int2* tiles, int ntiles, int sub, RKConst rk, int enforce,
+                             unsigned* status, cudaStream_t s, const void* D);
 template <typename T, typename SS>
 cudaError_t launch_face(const void* blocks, const int2* faces, int nfaces, int sub, RKConst rk, int enforce,
                         unsigned* status, cudaStream_t s);
 template <typename T, typename SS>
-cudaError_t launch_deriv(const void* blocks, const DerivItem* items, int nitems, int sub, void* D, long long dfs,
-                         int grid, cudaStream_t s, int occ);
+cudaError_t launch_deriv(const void* blocks, const DerivItem* items, int nitems, int sub, void* D, int slots,
+                         int region, int grid, cudaStream_t s, int occ);
 
 // out = E(in) on the metric / A~ fields; other fields copied.
 __global__ void k_enforce_copy(const double* __restrict__ in, double* __restrict__ out, long long n, long long fs) {
@@ -81,7 +81,7 @@ struct amss_adjoint {
   int ntiles = 0;
   int2* dfaces = nullptr;
   int nfaces = 0;
-  double* D = nullptr;                   // stencil terms (D_SLOTS x fs)
+  double* D = nullptr;                   // stencil terms (dterms)
   double* Db = nullptr;                  // their adjoints
   double* U = nullptr;                   // state (input of set_state / result of forward)
   double* U0 = nullptr;                  // enforced step start
@@ -109,6 +109,9 @@ struct amss_adjoint {
 namespace {
 
 size_t state_bytes(const amss_adjoint* a) { return (size_t)NFIELDS_BSSN * a->fs * sizeof(double); }
+
+// values of one array of stencil terms: whole tiles (stencil.cuh)
+size_t dterms(const amss_adjoint* a) { return (size_t)((a->npts + kDTile - 1) / kDTile) * kDTile * D_SLOTS; }
 
 int grid_of(long long n) {
   const long long b = (n + 127) / 128;
@@ -153,9 +156,8 @@ int fwd_step(amss_adjoint* a, const double* U0raw, double* Unew, double* Z0, dou
   for (int sub = 0; sub < 4; ++sub) {
     const StepBlock<double>* T = a->dtab + sub;
     double* D = Dsub ? Dsub[sub] : a->D;
-    AMSS_CK((launch_deriv<double, double>(T, a->ditems, a->nitems, sub, D, a->fs, std::min(a->nitems, 148 * 16), s, 0)));
-    AMSS_CK((launch_substep<double, double, false, true, false>(T, a->dtiles, a->ntiles, sub, rk, 0, a->dstatus,
-                                                              std::min(a->ntiles, 148 * 8), s, D, a->fs)));
+    AMSS_CK((launch_deriv<double, double>(T, a->ditems, a->nitems, sub, D, D_SLOTS, -1, std::min(a->nitems, 148 * 16), s, 0)));
+    AMSS_CK((launch_pointwise<double, double, false>(T, a->dtiles, a->ntiles, sub, rk, 0, a->dstatus, s, D)));
     AMSS_CK((launch_face<double, double>(T, a->dfaces, a->nfaces, sub, rk, 0, a->dstatus, s)));
     a->launches += 3;
     if (sub < 3) {
@@ -173,7 +175,7 @@ int rhs_vjp(amss_adjoint* a, int sub, const double* Xin, const double* Rbv, doub
   cudaStream_t s = a->stream;
   const StepBlock<double>* T = a->dtab + sub;
   if (!Dpre) {
-    AMSS_CK((launch_deriv<double, double>(T, a->ditems, a->nitems, sub, a->D, a->fs, std::min(a->nitems, 148 * 16), s, 0)));
+    AMSS_CK((launch_deriv<double, double>(T, a->ditems, a->nitems, sub, a->D, D_SLOTS, -1, std::min(a->nitems, 148 * 16), s, 0)));
     a->launches++;
   }
   a->host_adj.D = Dpre ? Dpre : a->D;
@@ -237,7 +239,7 @@ extern "C" amss_adjoint* amss_adjoint_create(const int ex[3], const double bbox[
       cudaMalloc(&a->dcoord, coord.size() * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&a->dtab, sizeof(a->host_tab)) != cudaSuccess ||
       cudaMalloc(&a->dadj, sizeof(AdjBlock)) != cudaSuccess ||
-      cudaMalloc(&a->D, (size_t)D_SLOTS * a->fs * sizeof(double)) != cudaSuccess ||
+      cudaMalloc(&a->D, dterms(a) * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&a->Db, (size_t)D_SLOTS * a->fs * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&a->H, a->fs * sizeof(double)) != cudaSuccess || cudaMalloc(&a->dloss, sizeof(double)) != cudaSuccess)
     return fail("amss_adjoint_create: device allocation failed");
@@ -343,7 +345,7 @@ static int loss_and_grad(amss_adjoint* a, double* loss, bool want_grad) {
   const int gw = 3;
   a->host_tab[0].tl[0] = a->U;   // stencil pass of U (substep-0 input)
   AMSS_CK(cudaMemcpyAsync(a->dtab, a->host_tab, sizeof(StepBlock<double>), cudaMemcpyHostToDevice, s));
-  AMSS_CK((launch_deriv<double, double>(a->dtab, a->ditems, a->nitems, 0, a->D, a->fs, std::min(a->nitems, 148 * 16), s, 0)));
+  AMSS_CK((launch_deriv<double, double>(a->dtab, a->ditems, a->nitems, 0, a->D, D_SLOTS, -1, std::min(a->nitems, 148 * 16), s, 0)));
   a->host_adj.D = a->D;
   a->host_adj.X = a->U;
   a->host_adj.Rb = nullptr;
@@ -380,7 +382,7 @@ static int reserve_segment(amss_adjoint* a) {
     AMSS_CK(cudaMalloc(&a->seg, (size_t)need * sb));
     a->seg_cap = need;
   }
-  const size_t dsz = (size_t)D_SLOTS * a->fs;
+  const size_t dsz = dterms(a);
   if (a->dseg_cap < 4 * a->ck) {
     if (a->Dseg) cudaFree(a->Dseg);
     a->Dseg = nullptr;
@@ -416,7 +418,7 @@ extern "C" int amss_adjoint_forward(amss_adjoint* a, double dt, int nsteps, int 
   // the steps of the last segment write their states (and stencil terms)
   // straight into the segment storage, which the reverse sweep starts from
   const long long m = (long long)NFIELDS_BSSN * a->fs;
-  const size_t dsz = (size_t)D_SLOTS * a->fs;
+  const size_t dsz = dterms(a);
   const int nlast = nck > 0 ? (nck - 1) * ck : 0;
   for (int n = 0; n < nsteps; ++n) {
     if (n % ck == 0) AMSS_CK(cudaMemcpyAsync(a->ckpt[n / ck], a->U, sb, cudaMemcpyDeviceToDevice, s));
@@ -449,7 +451,7 @@ extern "C" int amss_adjoint_backward(amss_adjoint* a, double* grad) {
   const int nck = (a->nsteps + a->ck - 1) / a->ck;
   if (int rc = reserve_segment(a)) return rc;   // allocated by the forward already
   auto st = [&](int slot) { return a->seg + (size_t)slot * m; };
-  const size_t dsz = (size_t)D_SLOTS * fs;
+  const size_t dsz = dterms(a);
   auto dst = [&](int t, int sub) { return a->Dseg ? a->Dseg + (size_t)(4 * t + sub) * dsz : nullptr; };
   // dL/dU at the final time
   double loss = 0;

@@ -39,8 +39,8 @@ struct AdjBlock {
   double d2s[3];
   long long npts;
   const double* X;    // linearization point (24 fields, stride b.fs)
-  const double* D;    // its stencil terms (slot stride dfs)
-  long long dfs;
+  const double* D;    // its stencil terms (tiles, stencil.cuh)
+  long long dfs;      // slot stride of their adjoints
   const double* Rb;   // adjoint of the right-hand side (24 fields)
   double* Xb;         // += adjoint of X
 };
@@ -56,6 +56,18 @@ struct SlotFieldTable {
 __device__ __forceinline__ int slot_field(int s) {
   constexpr SlotFieldTable t{};
   return t.f[s];
+}
+
+// D row of each slot
+struct SlotRowTable {
+  int r[D_SLOTS_Z4C];
+  constexpr SlotRowTable() : r() {
+    for (int s = 0; s < D_SLOTS_Z4C; ++s) r[s] = dl::row(s);
+  }
+};
+__device__ __forceinline__ int slot_row(int s) {
+  constexpr SlotRowTable t{};
+  return t.r[s];
 }
 
 // Scatter target of the Sommerfeld transpose: the field value at (i, j, k),
@@ -78,7 +90,7 @@ struct VjpIn {
   long long p;
   double hb;   // Hamiltonian-constraint adjoint (ham_vjp), output "field" 99
   __device__ __forceinline__ double c(int F) const { return A->X[F * A->b.fs + p]; }
-  __device__ __forceinline__ double d(int s) const { return A->D[s * A->dfs + p]; }
+  __device__ __forceinline__ double d(int s) const { return A->D[(p / kDTile * D_SLOTS + slot_row(s)) * kDTile + p % kDTile]; }
   __device__ __forceinline__ double rb(int F) const { return F == 99 ? hb : A->Rb[F * A->b.fs + p]; }
 };
 
@@ -86,7 +98,7 @@ struct VjpIn {
 // point) and the D-slot adjoints (stored, then gathered by k_stencil_gather_tiled).
 struct VjpStore {
   const AdjBlock* A;
-  double* Db;   // D-slot adjoints, same layout as D
+  double* Db;   // D-slot adjoints, slot s of point p at s * dfs + p
   long long p;
   __device__ __forceinline__ void cb(int F, double v) const { A->Xb[F * A->b.fs + p] = v; }
   __device__ __forceinline__ void db(int s, double v) const { Db[s * A->dfs + p] = v; }
@@ -121,7 +133,7 @@ __global__ void __launch_bounds__(128) k_rhs_vjp(const AdjBlock* __restrict__ bl
        p += (long long)gridDim.x * blockDim.x) {
     // this tile's rows meet the point function's one-by-one loads in L2
     const long long p0 = p - threadIdx.x;
-    prefetch_tile_rows(A.D, A.dfs, D_SLOTS, p0, A.npts);
+    prefetch_tile_rows(A.D + p0 * D_SLOTS, kDTile, D_SLOTS, 0, kDTile);
     prefetch_tile_rows(A.X, A.b.fs, NFIELDS_BSSN, p0, A.npts);
     prefetch_tile_rows(A.Rb, A.b.fs, NFIELDS_BSSN, p0, A.npts);
     int i, j, k;

@@ -64,7 +64,7 @@ __device__ __forceinline__ void finish_field(const P& q, const Coefs<T>& C, cons
                                              T bz, T add1, E& epi) {
   if constexpr (P::kPre) {
     // split form: the stencil pass stored advection + KO (0 where neither applies)
-    r = r + q.template dv<T>(doff(F) + dslots(F) - 1);
+    r = r + q.template dv<T, doff(F) + dslots(F) - 1>();
     epi.template put<F>(r);
   } else {
     if (g.lop) {
@@ -127,6 +127,7 @@ __device__ __forceinline__ unsigned bssn_rhs_point(const P& q, const Coefs<T>& C
   const T PI = T(3.141592653589793238462643383279502884);
   const int ord = G.ord;
 
+  phase<0>(q);
   // centre values; chi and alpha are read and shifted in FP64 (chi -> 0 near a
   // puncture, so chi+1 must be formed before rounding to T)
   using W = wide_t<T>;
@@ -173,6 +174,7 @@ __device__ __forceinline__ unsigned bssn_rhs_point(const P& q, const Coefs<T>& C
   const T alpn1 = (T)(Lap64 + W(1.0)), chin1 = (T)(chi64 + W(1.0));
   const T gxx = dxx + ONE, gyy = dyy + ONE, gzz = dzz + ONE;
 
+  phase<1>(q);
   // :152-160
   T betaxx, betaxy, betaxz, betayx, betayy, betayz, betazx, betazy, betazz;
   grad<T, F_BETAX>(q, C, ord, betaxx, betaxy, betaxz);
@@ -189,6 +191,7 @@ __device__ __forceinline__ unsigned bssn_rhs_point(const P& q, const Coefs<T>& C
   finish_field<T, F_BETAY>(q, C, G, FF * dtSfy, betax, betay, betaz, ZEO, epi);
   finish_field<T, F_BETAZ>(q, C, G, FF * dtSfz, betax, betay, betaz, ZEO, epi);
 
+  phase<2>(q);
   // :162-191
   T gxxx, gxxy, gxxz, gxyx, gxyy, gxyz, gxzx, gxzy, gxzz, gyyx, gyyy, gyyz, gyzx, gyzy, gyzz, gzzx, gzzy, gzzz;
   grad<T, F_GXX>(q, C, ord, gxxx, gxxy, gxxz);
@@ -198,6 +201,7 @@ __device__ __forceinline__ unsigned bssn_rhs_point(const P& q, const Coefs<T>& C
   grad<T, F_GYZ>(q, C, ord, gyzx, gyzy, gyzz);
   grad<T, F_GZZ>(q, C, ord, gzzx, gzzy, gzzz);
 
+  phase<3>(q);
   finish_field<T, F_GXX, Z4C>(q, C, G,
                          -TWO * alpn1 * Axx - F2o3 * gxx * div_beta +
                              TWO * (gxx * betaxx + gxy * betayx + gxz * betazx),
@@ -289,6 +293,7 @@ __device__ __forceinline__ unsigned bssn_rhs_point(const P& q, const Coefs<T>& C
   // :260-313 A~^ij and the Gamma-driver source without shift terms
   T Gamx_rhs, Gamy_rhs, Gamz_rhs;
   T Lapx, Lapy, Lapz;
+  phase<4>(q);
   grad<T, F_LAP>(q, C, ord, Lapx, Lapy, Lapz);
   {
     T Kx, Ky, Kz;
@@ -359,6 +364,7 @@ __device__ __forceinline__ unsigned bssn_rhs_point(const P& q, const Coefs<T>& C
                F1o3 * (gupxz * fxx + gupyz * fxy + gupzz * fxz) + gupxx * bz_xx + gupyy * bz_yy + gupzz * bz_zz +
                TWO * (gupxy * bz_xy + gupxz * bz_xz + gupyz * bz_yz);
   }
+  phase<5>(q);
   // :797-799 (GAUGE 0) and the advection / dissipation of Gam^i and B^i
   if constexpr (Z4C) {
     // Z4c_rhs.f90:1231-1233 constraint damping (B^i takes the undamped source)
@@ -400,6 +406,7 @@ __device__ __forceinline__ unsigned bssn_rhs_point(const P& q, const Coefs<T>& C
   gyzz = gxz * Gamxyz + gyz * Gamyyz + gzz * Gamzyz;
   gzzz = gxz * Gamxzz + gyz * Gamyzz + gzz * Gamzzz;
 
+  phase<6>(q);
   // :378-400 gup^kl d_k d_l g_ij, one metric component at a time
   T Rxx, Ryy, Rzz, Rxy, Rxz, Ryz;
   {
@@ -579,6 +586,7 @@ __device__ __forceinline__ unsigned bssn_rhs_point(const P& q, const Coefs<T>& C
     Rxx = Rxx_r; Ryy = Ryy_r; Rzz = Rzz_r; Rxy = Rxy_r; Rxz = Rxz_r; Ryz = Ryz_r;
   }
 
+  phase<7>(q);
   // :603-626 chi part of the Ricci tensor
   T fxx, fxy, fxz, fyy, fyz, fzz;
   hess<T, F_CHI>(q, C, ord, fxx, fxy, fxz, fyy, fyz, fzz);
@@ -635,6 +643,7 @@ __device__ __forceinline__ unsigned bssn_rhs_point(const P& q, const Coefs<T>& C
   fxz = fxz - Gamxxz * Lapx - Gamyxz * Lapy - Gamzxz * Lapz;
   fyz = fyz - Gamxyz * Lapx - Gamyyz * Lapy - Gamzyz * Lapz;
 
+  phase<8>(q);
   // :663-787 trK and A~_ij
   T trK_rhs = gupxx * fxx + gupyy * fyy + gupzz * fzz + TWO * (gupxy * fxy + gupxz * fxz + gupyz * fyz);
   // A~_il A~^l_j and its trace pieces, :729-746 (the same sums enter :669-694)

@@ -136,7 +136,8 @@ struct StepBlock {
   void* stage[2];     // stage buffers A and B (type of the stage storage)
   double* side[2];    // FP64 side slots (chi, alpha, beta^i) of stages A and B (mixed form only)
   double* K;          // RK accumulator (FP64)
-  long long doff;     // offset of this block's points in the level's D slots (split form)
+  long long doff;     // offset of this block's points in the level's scratch arrays (constraints, Psi4)
+  int dtile;          // first D tile of this block (split form)
   long long npts;
   int lev0;           // 1: Sommerfeld rule on the patch faces; 0: freeze them at u0
   int nf;             // evolved fields: 24 (BSSN) or 25 (Z4c, Theta last)

@@ -70,7 +70,7 @@ constexpr bool deriv_planes_fit(int w) {
 static_assert(deriv_planes_fit(kDerivMinEx), "plane buffer too small for a tile shape");
 
 // substep tile of the split form's pointwise pass
-constexpr int kPointwiseTile = 128;
+constexpr int kPointwiseTile = kDTile;
 // fewest planes of a z-slab of the stencil pass (each slab pays a 7-plane prologue)
 constexpr int kMinSlab = 8;
 
@@ -105,15 +105,11 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // A stencil term into D: written once here and read once by the pointwise
-// pass, so with AMSS_D_STREAMING bit 0 the store is marked evict-first
-// (st.global.cs) and leaves L2 to the fields the stencil pass re-reads.
+// pass: the store is marked evict-first (st.global.cs) and leaves L2 to the
+// fields the stencil pass re-reads.
 template <typename T>
 __device__ __forceinline__ void dstore(T* a, T v) {
-#if AMSS_D_STREAMING & 1
   __stcs(a, v);
-#else
-  *a = v;
-#endif
 }
 
 // The plane cells one thread fills, with their in-plane offsets and the x/y
@@ -273,7 +269,7 @@ __device__ __forceinline__ A lop_term(const FN& f, A b, A bd, int idx, int lo, i
 // of the D array.
 template <typename A, int KIND, bool ASYNC, typename T, typename S, typename SI>
 __device__ __forceinline__ void deriv_column(const StepBlock<T>& B, const S* src, const SI* in, const double* bsh,
-                                             int F, const DerivItem& it, T* D, long long dfs, A* ring) {
+                                             int F, const DerivItem& it, T* D, int slots, int region, A* ring) {
   const Coef<A>& C = pick<A>(B.C);
   const int ex0 = B.b.ex[0], ex1 = B.b.ex[1], ex2 = B.b.ex[2];
   const int x0 = it.x0, y0 = it.y0, k0 = it.k0;
@@ -292,8 +288,11 @@ __device__ __forceinline__ void deriv_column(const StepBlock<T>& B, const S* src
   // the diagonal metric is advected as g = d + 1 (bssn_rhs.f90:948-953) in FP64,
   // bit-faithful to the reference; FP32 advects d (the constant drops out)
   const A add1 = (sizeof(A) == 8 && (F == F_GXX || F == F_GYY || F == F_GZZ)) ? A(1) : A(0);
-  const int o = doff(F);
-  T* d = D + B.doff;
+  // D rows of the field's terms, and the point's entry in its tile order
+  const int og = dl::g(F) * kDTile, oh = dl::h(F) * kDTile, oa = dl::a(F) * kDTile;
+  const int rx = region < 0 ? 0 : B.rlo[region][0], ry = region < 0 ? 0 : B.rlo[region][1];
+  const int rz = region < 0 ? 0 : B.rlo[region][2];
+  const int rn0 = region < 0 ? ex0 : B.rn[region][0], rn1 = region < 0 ? ex1 : B.rn[region][1];
   const int own = (lj < H ? lj + 3 : 3) * DSX + (li + 3);   // idle threads read a valid cell
 
   // ASYNC: cp.async fills the ring where the source needs no conversion (six
@@ -409,6 +408,8 @@ __device__ __forceinline__ void deriv_column(const StepBlock<T>& B, const S* src
     if (mine && !on_face) {
       const PointGates G = point_gates(B.b, i, j, k);
       const long long p = i + (long long)j * ex0 + (long long)k * ex0 * ex1;
+      const long long dq = (i - rx) + (long long)rn0 * ((j - ry) + (long long)rn1 * (k - rz));
+      T* d = D + (B.dtile + dq / kDTile) * ((long long)slots * kDTile) + dq % kDTile;
       auto X = [&](int dd) { return qk[dd]; };
       auto Y = [&](int dd) { return qk[dd * DSX]; };
       auto Z = [&](int dd) { return c[3 + dd]; };
@@ -423,9 +424,9 @@ __device__ __forceinline__ void deriv_column(const StepBlock<T>& B, const S* src
           else { gx = dx2(qk); gy = dy2(qk); }
           gz = C.d2[2] * (-Z(-1) + Z(1));
         }
-        dstore(d + (o + 0) * dfs + p, (T)gx);
-        dstore(d + (o + 1) * dfs + p, (T)gy);
-        dstore(d + (o + 2) * dfs + p, (T)gz);
+        dstore(d + og + 0 * kDTile, (T)gx);
+        dstore(d + og + 1 * kDTile, (T)gy);
+        dstore(d + og + 2 * kDTile, (T)gz);
       }
       if constexpr (KIND == 0) {
         A hxx = A(0), hxy = A(0), hxz = A(0), hyy = A(0), hyz = A(0), hzz = A(0);
@@ -449,12 +450,12 @@ __device__ __forceinline__ void deriv_column(const StepBlock<T>& B, const S* src
           hxz = C.d2[2] * (-fx2[0] + fx2[2]);
           hyz = C.d2[2] * (-fy2[0] + fy2[2]);
         }
-        dstore(d + (o + 3) * dfs + p, (T)hxx);
-        dstore(d + (o + 4) * dfs + p, (T)hxy);
-        dstore(d + (o + 5) * dfs + p, (T)hxz);
-        dstore(d + (o + 6) * dfs + p, (T)hyy);
-        dstore(d + (o + 7) * dfs + p, (T)hyz);
-        dstore(d + (o + 8) * dfs + p, (T)hzz);
+        dstore(d + oh + 0 * kDTile, (T)hxx);
+        dstore(d + oh + 1 * kDTile, (T)hxy);
+        dstore(d + oh + 2 * kDTile, (T)hxz);
+        dstore(d + oh + 3 * kDTile, (T)hyy);
+        dstore(d + oh + 4 * kDTile, (T)hyz);
+        dstore(d + oh + 5 * kDTile, (T)hzz);
       }
       A adv = A(0);
       if (G.lop) {
@@ -483,7 +484,7 @@ __device__ __forceinline__ void deriv_column(const StepBlock<T>& B, const S* src
                kodiv(ko_sum_rn<A, false>(Z), C, 2);
         adv = adv + C.ko * ks;
       }
-      dstore(d + (o + dslots(F) - 1) * dfs + p, (T)adv);
+      dstore(d + oa, (T)adv);
     }
     // slide the register windows
 #pragma unroll
@@ -514,7 +515,7 @@ __device__ __forceinline__ void deriv_column(const StepBlock<T>& B, const S* src
 template <typename T, typename SI, int MINB>
 __global__ void __launch_bounds__(DTHREADS, MINB) k_deriv(const StepBlock<T>* __restrict__ blocks,
                                                       const DerivItem* __restrict__ items, int nitems, int sub,
-                                                      T* __restrict__ D, long long dfs) {
+                                                      T* __restrict__ D, int slots, int region) {
   extern __shared__ __align__(16) unsigned char smem[];
   // the two-CTA form fills its ring by cp.async; the forms with more CTAs keep
   // the register path, whose smaller ring leaves L1 to their spills
@@ -533,16 +534,16 @@ __global__ void __launch_bounds__(DTHREADS, MINB) k_deriv(const StepBlock<T>* __
         // wide fields of the mixed form: FP64 source (state, or the FP64 side stage) and arithmetic
         const double* src = sizeof(SI) == 4 ? B.side[sub == 2 ? 1 : 0] + side_slot(F) * fs
                                             : (const double*)in + F * fs;
-        deriv_column<double, 0, kAsyncForm>(B, src, in, bsh, F, it, D, dfs, reinterpret_cast<double*>(smem));
+        deriv_column<double, 0, kAsyncForm>(B, src, in, bsh, F, it, D, slots, region, reinterpret_cast<double*>(smem));
         __syncthreads();
         continue;
       }
     }
     const SI* src = in + F * fs;
     switch (dkind(F)) {
-      case 0: deriv_column<T, 0, kAsyncForm>(B, src, in, bsh, F, it, D, dfs, reinterpret_cast<T*>(smem)); break;
-      case 1: deriv_column<T, 1, kAsyncForm>(B, src, in, bsh, F, it, D, dfs, reinterpret_cast<T*>(smem)); break;
-      default: deriv_column<T, 2, kAsyncForm>(B, src, in, bsh, F, it, D, dfs, reinterpret_cast<T*>(smem)); break;
+      case 0: deriv_column<T, 0, kAsyncForm>(B, src, in, bsh, F, it, D, slots, region, reinterpret_cast<T*>(smem)); break;
+      case 1: deriv_column<T, 1, kAsyncForm>(B, src, in, bsh, F, it, D, slots, region, reinterpret_cast<T*>(smem)); break;
+      default: deriv_column<T, 2, kAsyncForm>(B, src, in, bsh, F, it, D, slots, region, reinterpret_cast<T*>(smem)); break;
     }
     __syncthreads();
   }
@@ -552,5 +553,25 @@ __global__ void __launch_bounds__(DTHREADS, MINB) k_deriv(const StepBlock<T>* __
 // the two-CTA form (cp.async ring) and the others (register path).
 constexpr size_t kDerivSmemLow = (size_t)(AMSS_DERIV_ASYNC ? DRING_ASYNC : DRING) * DPLANE * sizeof(double);
 constexpr size_t kDerivSmem = (size_t)DRING * DPLANE * sizeof(double);
+
+// Stencil pass launcher: substep 0 reads the FP64 state, 1-3 the stages;
+// region: the D order of the points (-1: whole arrays, else StepBlock::rlo);
+// occ selects the compiled occupancy (0: two resident CTAs, 1: more).
+template <typename T, typename SS>
+cudaError_t launch_deriv(const void* blocks, const DerivItem* items, int nitems, int sub, void* D, int slots,
+                         int region, int grid, cudaStream_t s, int occ) {
+  const StepBlock<T>* bl = (const StepBlock<T>*)blocks;
+  // both < 48 KB: no opt-in attribute needed
+  const size_t smem = occ ? kDerivSmem : kDerivSmemLow;
+  constexpr int hi = sizeof(T) == 8 ? AMSS_DERIV_MINB_F64 : AMSS_DERIV_MINB_F32;
+  if (sub == 0) {
+    if (occ) k_deriv<T, double, hi><<<grid, DTHREADS, smem, s>>>(bl, items, nitems, sub, (T*)D, slots, region);
+    else k_deriv<T, double, kDerivMinbLow><<<grid, DTHREADS, smem, s>>>(bl, items, nitems, sub, (T*)D, slots, region);
+  } else {
+    if (occ) k_deriv<T, SS, hi><<<grid, DTHREADS, smem, s>>>(bl, items, nitems, sub, (T*)D, slots, region);
+    else k_deriv<T, SS, kDerivMinbLow><<<grid, DTHREADS, smem, s>>>(bl, items, nitems, sub, (T*)D, slots, region);
+  }
+  return cudaGetLastError();
+}
 
 }  // namespace amss

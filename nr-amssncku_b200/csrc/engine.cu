@@ -30,15 +30,18 @@ template <typename T>
 Coef<T> make_coef(const double dx[3], double eps);
 void block_faces(const int ex[3], const double* X, const double* Y, const double* Z, const double bbox[6],
                  int symmetry, int* face_mask, int* lowsym_mask);
-template <typename T, typename SS, bool SYMM, bool SPLIT, bool Z4C>
+template <typename T, typename SS, bool SYMM>
 cudaError_t launch_substep(const void* blocks, const int2* tiles, int ntiles, int sub, RKConst rk, int enforce,
-                           unsigned* status, int grid, cudaStream_t s, const void* D, long long dfs);
+                           unsigned* status, int grid, cudaStream_t s);
+template <typename T, typename SS, bool Z4C>
+cudaError_t launch_pointwise(const void* blocks, const int2* tiles, int ntiles, int sub, RKConst rk, int enforce,
+                             unsigned* status, cudaStream_t s, const void* D);
 template <typename T, typename SS>
 cudaError_t launch_face(const void* blocks, const int2* faces, int nfaces, int sub, RKConst rk, int enforce,
                         unsigned* status, cudaStream_t s);
 template <typename T, typename SS>
-cudaError_t launch_deriv(const void* blocks, const DerivItem* items, int nitems, int sub, void* D, long long dfs,
-                         int grid, cudaStream_t s, int occ);
+cudaError_t launch_deriv(const void* blocks, const DerivItem* items, int nitems, int sub, void* D, int slots,
+                         int region, int grid, cudaStream_t s, int occ);
 cudaError_t launch_enforce(long long n, long long fs, double* g, double* a, cudaStream_t s);
 template <typename T>
 cudaError_t launch_constraints(const void* table, const int2* tiles, int ntiles, int tile_pts, bool symm,
@@ -331,11 +334,14 @@ static int build_table(amss_engine* e, ELevel& L, int level) {
   std::vector<int2> faces;
   std::vector<DerivItem> items;
   long long doff = 0;
+  int dtile = 0;
   for (size_t m = 0; m < L.own.size(); ++m) {
     EBlock& b = e->blocks[L.own[m]];
     StepBlock<T> s{};
     s.doff = doff;
     doff += b.fs;
+    s.dtile = dtile;
+    dtile += (int)((b.npts + kDTile - 1) / kDTile);
     s.b.ex[0] = b.ex[0]; s.b.ex[1] = b.ex[1]; s.b.ex[2] = b.ex[2];
     s.b.fs = b.fs;
     s.b.X = b.dX; s.b.Y = b.dX + b.ex[0]; s.b.Z = b.dX + b.ex[0] + b.ex[1];
@@ -442,6 +448,7 @@ static int build_table(amss_engine* e, ELevel& L, int level) {
     }
   }
   L.dfs = doff;
+  L.dtiles_n = dtile;
   L.nditems = (int)items.size();
   if (tab.empty()) return 0;   // a rank without blocks on this level: no step tables
   AMSS_CK(cudaMalloc(&L.ditems, items.size() * sizeof(DerivItem)));
@@ -594,7 +601,7 @@ extern "C" int amss_engine_commit(amss_engine* e) {
   }
   if (e->prm.kernel == 0) {
     long long mx = 0;
-    for (auto& kv : e->levels) mx = std::max(mx, kv.second.dfs);
+    for (auto& kv : e->levels) mx = std::max(mx, (long long)kv.second.dtiles_n * kDTile);
     const int slots = e->nf == NFIELDS_Z4C ? D_SLOTS_Z4C : D_SLOTS;
     if (mx) AMSS_CK(cudaMalloc(&e->D, (size_t)mx * slots * (mixed ? sizeof(float) : sizeof(double))));
   }
@@ -797,26 +804,26 @@ static int step_level_impl(amss_engine* e, int level, double dt, bool fin = fals
       e->launches++;
     }
     if (split && nditems) {
+      const int slots = e->nf == NFIELDS_Z4C ? D_SLOTS_Z4C : D_SLOTS, region = reg ? 0 : own ? 1 : -1;
       const cudaError_t ed =
-          mixed ? launch_deriv<float, float>(L.dtable, ditems, nditems, sub, e->D, L.dfs, dgrid, e->stream, L.docc)
-                : launch_deriv<double, double>(L.dtable, ditems, nditems, sub, e->D, L.dfs, dgrid, e->stream, L.docc);
+          mixed ? launch_deriv<float, float>(L.dtable, ditems, nditems, sub, e->D, slots, region, dgrid, e->stream, L.docc)
+                : launch_deriv<double, double>(L.dtable, ditems, nditems, sub, e->D, slots, region, dgrid, e->stream, L.docc);
       AMSS_CK(ed);
       e->launches++;
     }
-#define AMSS_SUB(T, SY, SP, Z) \
-    launch_substep<T, T, SY, SP, Z>(L.dtable, tiles, ntiles, sub, rk, enf, e->dstatus, grid, e->stream, e->D, L.dfs)
-    if (ntiles == 0)
+    if (ntiles == 0) {
       err = cudaSuccess;
-    else if (e->nf == NFIELDS_Z4C)   // split form only (checked at create)
-      err = mixed ? (L.symm ? AMSS_SUB(float, true, true, true) : AMSS_SUB(float, false, true, true))
-                  : (L.symm ? AMSS_SUB(double, true, true, true) : AMSS_SUB(double, false, true, true));
-    else if (mixed)
-      err = split ? (L.symm ? AMSS_SUB(float, true, true, false) : AMSS_SUB(float, false, true, false))
-                  : (L.symm ? AMSS_SUB(float, true, false, false) : AMSS_SUB(float, false, false, false));
-    else
-      err = split ? (L.symm ? AMSS_SUB(double, true, true, false) : AMSS_SUB(double, false, true, false))
-                  : (L.symm ? AMSS_SUB(double, true, false, false) : AMSS_SUB(double, false, false, false));
+    } else if (split) {
+#define AMSS_PW(T, Z) launch_pointwise<T, T, Z>(L.dtable, tiles, ntiles, sub, rk, enf, e->dstatus, e->stream, e->D)
+      if (e->nf == NFIELDS_Z4C) err = mixed ? AMSS_PW(float, true) : AMSS_PW(double, true);
+      else err = mixed ? AMSS_PW(float, false) : AMSS_PW(double, false);
+#undef AMSS_PW
+    } else {   // BSSN only (checked at create)
+#define AMSS_SUB(T, SY) launch_substep<T, T, SY>(L.dtable, tiles, ntiles, sub, rk, enf, e->dstatus, grid, e->stream)
+      err = mixed ? (L.symm ? AMSS_SUB(float, true) : AMSS_SUB(float, false))
+                  : (L.symm ? AMSS_SUB(double, true) : AMSS_SUB(double, false));
 #undef AMSS_SUB
+    }
     AMSS_CK(err);
     if (ntiles) e->launches++;
     // Outer faces.  Level 0: the Sommerfeld rule at every substep.  A refined

@@ -133,29 +133,72 @@ static_assert(doff(24) == D_SLOTS, "D slot layout");
 constexpr int D_SLOTS_Z4C = D_SLOTS + 4;
 static_assert(doff(F_TZ) == D_SLOTS && doff(F_TZ + 1) == D_SLOTS_Z4C, "Z4c D slot layout");
 
-#ifndef AMSS_D_STREAMING   // the D array marked evict-first: bit 0 its stores, bit 1 its loads
-#define AMSS_D_STREAMING 3
-#endif
-
-// Accessor of the pointwise pass: centre values from the stage input (Pt),
-// stencil terms from the D array written by the stencil pass.
-template <typename SI, bool SYMM, typename DT>
-struct DPt : Pt<SI, SYMM> {
-  static constexpr bool kPre = true;
-  const DT* __restrict__ d;   // slot 0 of this point's block (add slot * dfs + p)
-  long long dfs;              // slot stride
-  template <typename T>
-  __device__ __forceinline__ T dv(int slot) const {
-#if AMSS_D_STREAMING & 2
-    return (T)__ldcs(d + slot * dfs + this->p);
-#else
-    return (T)__ldg(d + slot * dfs + this->p);
-#endif
+// Layout of the D array: tiles of kDTile points (the pointwise pass's tiles, in
+// its order), a tile's rows (one stencil term of its points each) contiguous.
+// The rows come in the order in which the pointwise pass's phases use them
+// (pointwise.cuh), so that a phase's terms are one run of memory:
+//   phase 1: gradients of beta and chi, adv of chi, alpha, beta
+//   phase 2: metric gradients        phase 3: metric adv
+//   phase 4: gradients of alpha and K, Hessians of beta
+//   phase 5: adv of Gamma and B, gradients of Gamma
+//   phase 6: metric Hessians         phase 7: Hessians of chi and alpha
+//   phase 8: adv of A~ and K;        then Theta (Z4c): gradient, adv
+constexpr int kDTile = 128;
+namespace dl {
+__host__ __device__ constexpr int first(int ph) {   // first row of a phase
+  constexpr int f[10] = {0, 0, 17, 35, 41, 65, 80, 116, 128, 135};
+  return f[ph];
+}
+constexpr int kTheta = D_SLOTS;
+__host__ __device__ constexpr bool is_g(int F) { return F >= F_GXX && F <= F_GZZ; }
+__host__ __device__ constexpr bool is_a(int F) { return F >= F_AXX && F <= F_AZZ; }
+// first row of a field's gradient, of its Hessian, and the row of its adv
+__host__ __device__ constexpr int g(int F) {
+  return F >= F_BETAX && F <= F_BETAZ ? 3 * (F - F_BETAX) : F == F_CHI ? 9 : is_g(F) ? first(2) + 3 * (F - F_GXX)
+         : F == F_LAP ? first(4) : F == F_TRK ? first(4) + 3 : F == F_TZ ? kTheta : first(5) + 6 + 3 * (F - F_GAMX);
+}
+__host__ __device__ constexpr int h(int F) {
+  return F >= F_BETAX && F <= F_BETAZ ? first(4) + 6 + 6 * (F - F_BETAX) : is_g(F) ? first(6) + 6 * (F - F_GXX)
+         : F == F_CHI ? first(7) : first(7) + 6;
+}
+__host__ __device__ constexpr int a(int F) {
+  return F == F_CHI ? 12 : F == F_LAP ? 13 : F >= F_BETAX && F <= F_BETAZ ? 14 + (F - F_BETAX)
+         : is_g(F) ? first(3) + (F - F_GXX) : F >= F_GAMX && F <= F_GAMZ ? first(5) + (F - F_GAMX)
+         : F >= F_DTSFX && F <= F_DTSFZ ? first(5) + 3 + (F - F_DTSFX) : is_a(F) ? first(8) + (F - F_AXX)
+         : F == F_TRK ? first(8) + 6 : kTheta + 3;
+}
+// row of a slot (doff(F) + component)
+__host__ __device__ constexpr int row(int slot) {
+  int F = 0;
+  while (doff(F + 1) <= slot) ++F;
+  const int c = slot - doff(F), n = dslots(F);
+  return c == n - 1 ? a(F) : (c < 3 ? g(F) + c : h(F) + c - 3);
+}
+constexpr bool rows_distinct() {
+  bool seen[D_SLOTS_Z4C] = {};
+  for (int s = 0; s < D_SLOTS_Z4C; ++s) {
+    const int r = row(s);
+    if (r < 0 || r >= D_SLOTS_Z4C || seen[r] || (s < D_SLOTS) != (r < D_SLOTS)) return false;
+    seen[r] = true;
   }
-};
+  return true;
+}
+static_assert(rows_distinct(), "every slot has a row of its own");
+}  // namespace dl
 
 template <int D>
 __device__ __forceinline__ constexpr int ax(int d) { return D == d ? 1 : 0; }
+
+// The point function enters phase N of its inputs (pointwise.cuh): accessors
+// that stage them wait here, the others have nothing to do.
+template <typename P, typename = void>
+struct has_phases : std::false_type {};
+template <typename P>
+struct has_phases<P, std::void_t<decltype(&P::template phase<0>)>> : std::true_type {};
+template <int N, typename P>
+__device__ __forceinline__ void phase(const P& q) {
+  if constexpr (has_phases<P>::value) q.template phase<N>();
+}
 
 // ---- first derivatives (fderivs), one direction D ---------------------------
 // 4th order: d12 * (f(-2) - 8 f(-1) + 8 f(+1) - f(+2))
@@ -189,7 +232,7 @@ __device__ __forceinline__ void grad_a(const P& q, const Coef<T>& C, int ord, T&
 template <typename T, int F, typename P>
 __device__ __forceinline__ void grad(const P& q, const Coefs<T>& C, int ord, T& fx, T& fy, T& fz) {
   if constexpr (P::kPre) {
-    fx = q.template dv<T>(doff(F) + 0); fy = q.template dv<T>(doff(F) + 1); fz = q.template dv<T>(doff(F) + 2);
+    fx = q.template dv<T, doff(F) + 0>(); fy = q.template dv<T, doff(F) + 1>(); fz = q.template dv<T, doff(F) + 2>();
   } else {
     using A = std::conditional_t<wide_field<F>(), double, T>;
     A ax, ay, az;
@@ -256,9 +299,9 @@ template <typename T, int F, typename P>
 __device__ __forceinline__ void hess(const P& q, const Coefs<T>& C, int ord, T& fxx, T& fxy, T& fxz, T& fyy,
                                      T& fyz, T& fzz) {
   if constexpr (P::kPre) {
-    const int o = doff(F) + 3;
-    fxx = q.template dv<T>(o); fxy = q.template dv<T>(o + 1); fxz = q.template dv<T>(o + 2);
-    fyy = q.template dv<T>(o + 3); fyz = q.template dv<T>(o + 4); fzz = q.template dv<T>(o + 5);
+    constexpr int o = doff(F) + 3;
+    fxx = q.template dv<T, o>(); fxy = q.template dv<T, o + 1>(); fxz = q.template dv<T, o + 2>();
+    fyy = q.template dv<T, o + 3>(); fyz = q.template dv<T, o + 4>(); fzz = q.template dv<T, o + 5>();
   } else {
     using A = std::conditional_t<wide_field<F>(), double, T>;
     A a[6];

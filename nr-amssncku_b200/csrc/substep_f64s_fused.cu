@@ -3,6 +3,6 @@
 #include "substep_impl.cuh"
 
 namespace amss {
-template cudaError_t launch_substep<double, double, true, false, false>(const void*, const int2*, int, int, RKConst, int,
-                                                       unsigned*, int, cudaStream_t, const void*, long long);
+template cudaError_t launch_substep<double, double, true>(const void*, const int2*, int, int, RKConst, int, unsigned*, int,
+                                                cudaStream_t);
 }  // namespace amss

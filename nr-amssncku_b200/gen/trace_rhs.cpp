@@ -98,8 +98,9 @@ struct RecPt {
     if (it == cin.end()) it = cin.emplace(F, trace::push('c', F, -1)).first;
     return Rec::of(it->second);
   }
-  template <typename U>
-  U dv(int slot) const {
+  template <typename U, int SLOT>
+  U dv() const {
+    const int slot = SLOT;
     auto it = din.find(slot);
     if (it == din.end()) it = din.emplace(slot, trace::push('d', slot, -1)).first;
     return Rec::of(it->second);
