@@ -61,86 +61,94 @@ __device__ __constant__ double kProlongW[6] = {7.7e1 / 8.192e3, -6.93e2 / 8.192e
 // the right child of k = g >> 1 (coarse k-2..k+3, weights C1..C6), g even
 // the left child (coarse k-3..k+2, weights C6..C1).
 //
-// One thread takes one field of a run of kProlongRun fine cells along x that
-// starts at an even index (cells outside the box are skipped).  The cells of a
-// run share their y and z weights, so the z-then-y reduction of each coarse x
-// column the run reads is formed once (14 columns for 16 cells instead of 6
-// per cell) and the x sums of the cells reuse it: the same operations in the same
-// order as the cell-by-cell form.  Tiles count (field, run) units, field-major
-// within a box, not cells.
-__global__ void k_amr_prolong(const AmrBlock* __restrict__ blocks, const AmrBox* __restrict__ boxes,
-                              const int2* __restrict__ tiles, int ntiles, int from_temp, unsigned* status) {
+// The pass is bound by its loads: one thread a run of fine cells read 31
+// values a cell from lines of its own (208 us a call of the 48^3 boxes).  A
+// lane takes one coarse x column instead, so that a warp's loads are
+// consecutive, and the four (y, z) rows of fine cells over one coarse cell
+// share the column's 7 x 7 values: it reduces them over z and y for each row;
+// the x sums of its coarse cell's children then read the columns of the
+// neighbouring lanes by shuffle, in the reference's order of operations.
+// 79 us now.  A unit is (field, z pair, y pair, x piece): a segment of
+// `seg` lanes, whose inner seg - 6 have children to write.  Boxes a few cells
+// wide pack three segments of 10 lanes, or two of 16, into a warp.
+__global__ void __launch_bounds__(128) k_amr_prolong(const AmrBlock* __restrict__ blocks,
+                                                     const AmrBox* __restrict__ boxes, const int2* __restrict__ tiles,
+                                                     int ntiles, int from_temp, unsigned* status) {
+  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int2 tile = tiles[t];
     const AmrBox& bx = boxes[tile.x];
-    const int nrx = prolong_runs_x(bx.lo[0], bx.n[0]);
-    const int nru = nrx * bx.n[1] * bx.n[2];
+    const ProlongUnits U(bx);
     const AmrBlock& D = blocks[bx.dst];
-    const int uu = tile.y + threadIdx.x;
-    if (uu >= nru * D.nf) continue;
-    const int f = uu / nru, u = uu - f * nru;
-    const int xs = (bx.lo[0] & ~1) + (u % nrx) * kProlongRun;   // even first fine x of the run
-    const int gy = bx.lo[1] + (u / nrx) % bx.n[1], gz = bx.lo[2] + u / (nrx * bx.n[1]);
-    const int xlo = bx.lo[0], xhi = bx.lo[0] + bx.n[0];
     const AmrBlock& S = blocks[bx.src];
-    const bool ry = (gy & 1) == 0, rz = (gz & 1) == 0;
-    const int sy0 = ry ? (gy >> 1) - 3 : (gy >> 1) - 2;
-    const int sz0 = rz ? (gz >> 1) - 3 : (gz >> 1) - 2;
-    const int cx0 = (xs >> 1) - 3;   // coarse x column of T[0]
-    // every source cell of the run, and every destination cell, must exist
-    const int first = xs < xlo ? xlo : xs, last = (xs + kProlongRun < xhi ? xs + kProlongRun : xhi) - 1;
-    const int c_first = (first & 1) ? (first >> 1) - 2 : (first >> 1) - 3;
-    const int c_last = ((last & 1) ? (last >> 1) - 2 : (last >> 1) - 3) + 5;
-    if (!amr_inside(D, first, gy, gz) || !amr_inside(D, last, gy, gz) || !amr_inside(S, c_first, sy0, sz0) ||
-        !amr_inside(S, c_last, sy0 + 5, sz0 + 5)) {
+    const int s = lane / U.seg, l = lane - s * U.seg;   // segment of the warp, lane in it
+    const int uu = tile.y + warp * U.per_warp + s;
+    const bool on = s < U.per_warp && uu < U.count * D.nf;
+    const int f = on ? uu / U.count : 0, u = on ? uu - f * U.count : 0;
+    const int m0 = U.c0[0] + (u % U.nx) * (U.seg - 6);       // first coarse cell of the piece
+    const int cy = U.c0[1] + (u / U.nx) % U.ny, cz = U.c0[2] + u / (U.nx * U.ny);
+    const int cx = m0 - 3 + l;                               // this lane's column
+    int lo[3], hi[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) { lo[d] = bx.lo[d]; hi[d] = bx.lo[d] + bx.n[d]; }
+    // which rows and cells exist, and the coarse values they read
+    const int mine = m0 + U.seg - 6 < U.c0[0] + U.nc ? m0 + U.seg - 6 : U.c0[0] + U.nc;   // end of the piece
+    const int fx0 = 2 * m0 < lo[0] ? lo[0] : 2 * m0, fx1 = 2 * mine < hi[0] ? 2 * mine : hi[0];   // its fine cells
+    const bool ye = 2 * cy >= lo[1], yo = 2 * cy + 1 < hi[1], ze = 2 * cz >= lo[2], zo = 2 * cz + 1 < hi[2];
+    const int xa = (fx0 & 1) ? (fx0 >> 1) - 2 : (fx0 >> 1) - 3, xb = (fx1 >> 1) + 2;
+    const int ra = ye ? 0 : 1, rb = yo ? 6 : 5, qa = ze ? 0 : 1, qb = zo ? 6 : 5;
+    bool ok = on;
+    if (on && (!amr_inside(D, fx0, ye ? 2 * cy : 2 * cy + 1, ze ? 2 * cz : 2 * cz + 1) ||
+               !amr_inside(D, fx1 - 1, yo ? 2 * cy + 1 : 2 * cy, zo ? 2 * cz + 1 : 2 * cz) ||
+               !amr_inside(S, xa, cy - 3 + ra, cz - 3 + qa) || !amr_inside(S, xb, cy - 3 + rb, cz - 3 + qb))) {
       atomicOr(status, ST_BAD_ARG);
-      continue;
+      ok = false;
     }
-    const double* src = from_temp ? S.K : amr_state(S);
-    const long long sy = S.ex[0], sz = (long long)S.ex[0] * S.ex[1];
-    double wy[6], wz[6];
+    // T[2 zr + yr]: the column reduced over z and y for the row of fine parity (yr, zr)
+    double T[4] = {0.0, 0.0, 0.0, 0.0};
+    if (ok && cx >= xa && cx <= xb) {
+      const double* q = (from_temp ? S.K : amr_state(S)) + f * S.fs + amr_idx(S, cx, cy - 3, cz - 3);
+      const long long sy = S.ex[0], sz = (long long)S.ex[0] * S.ex[1];
 #pragma unroll
-    for (int m = 0; m < 6; ++m) {
-      wy[m] = kProlongW[ry ? 5 - m : m];
-      wz[m] = kProlongW[rz ? 5 - m : m];
-    }
-    double* dst = amr_state(D);
-    const long long od0 = amr_idx(D, xs, gy, gz);
-    // columns the run reads: T[c] for coarse x = cx0 + c, c in [c_first - cx0, c_last - cx0]
-    const int cb = c_first - cx0, ce = c_last - cx0;
-    {
-      const double* q = src + f * S.fs;
-      double T[kProlongRun / 2 + 6];
+      for (int r = 0; r < 7; ++r) {
+        if (r < ra || r > rb) continue;
+        double v[7];
 #pragma unroll
-      for (int c = 0; c < kProlongRun / 2 + 6; ++c) {
-        T[c] = 0.0;
-        if (c < cb || c > ce) continue;
-        const long long base = amr_idx(S, cx0 + c, sy0, sz0);
-        double t1 = 0.0;
+        for (int m = 0; m < 7; ++m) v[m] = m >= qa && m <= qb ? q[r * sy + m * sz] : 0.0;
+        double te = __dmul_rn(kProlongW[5], v[0]), to = __dmul_rn(kProlongW[0], v[1]);
 #pragma unroll
-        for (int b = 0; b < 6; ++b) {
-          const double* r = q + base + b * sy;
-          double t2 = __dmul_rn(wz[0], r[0]);
-#pragma unroll
-          for (int m = 1; m < 6; ++m) t2 = __dadd_rn(t2, __dmul_rn(wz[m], r[m * sz]));
-          t1 = b == 0 ? __dmul_rn(wy[0], t2) : __dadd_rn(t1, __dmul_rn(wy[b], t2));
+        for (int m = 1; m < 6; ++m) {
+          te = __dadd_rn(te, __dmul_rn(kProlongW[5 - m], v[m]));
+          to = __dadd_rn(to, __dmul_rn(kProlongW[m], v[m + 1]));
         }
-        T[c] = t1;
+        if (r < 6) {   // left child in y: rows 0 .. 5, weights C6 .. C1
+          T[0] = r == 0 ? __dmul_rn(kProlongW[5], te) : __dadd_rn(T[0], __dmul_rn(kProlongW[5 - r], te));
+          T[2] = r == 0 ? __dmul_rn(kProlongW[5], to) : __dadd_rn(T[2], __dmul_rn(kProlongW[5 - r], to));
+        }
+        if (r > 0) {   // right child: rows 1 .. 6, weights C1 .. C6
+          T[1] = r == 1 ? __dmul_rn(kProlongW[0], te) : __dadd_rn(T[1], __dmul_rn(kProlongW[r - 1], te));
+          T[3] = r == 1 ? __dmul_rn(kProlongW[0], to) : __dadd_rn(T[3], __dmul_rn(kProlongW[r - 1], to));
+        }
       }
+    }
+    // x sums of the lane's coarse cell: its children 2 cx and 2 cx + 1
+    double* dst = amr_state(D) + f * D.fs;
+    const bool wl = ok && l >= 3 && l < U.seg - 3 && 2 * cx >= fx0 && 2 * cx < fx1;
+    const bool wr = ok && l >= 3 && l < U.seg - 3 && 2 * cx + 1 >= fx0 && 2 * cx + 1 < fx1;
 #pragma unroll
-      for (int i = 0; i < kProlongRun; ++i) {
-        const int gx = xs + i;
-        if (gx < xlo || gx >= xhi) continue;
-        // even i: left child, coarse columns i/2 .. i/2 + 5 of T with weights C6..C1;
-        // odd i: right child, columns i/2 + 1 .. i/2 + 6 with C1..C6
-        const int c0 = (i & 1) ? i / 2 + 1 : i / 2;
-        double v = 0.0;
+    for (int m = 0; m < 4; ++m) {
+      double vl = 0.0, vr = 0.0;
 #pragma unroll
-        for (int a = 0; a < 6; ++a) {
-          const double w = kProlongW[(i & 1) ? a : 5 - a];
-          v = a == 0 ? __dmul_rn(w, T[c0]) : __dadd_rn(v, __dmul_rn(w, T[c0 + a]));
-        }
-        dst[f * D.fs + od0 + i] = v;
+      for (int a = 0; a < 7; ++a) {
+        const double c = __shfl_sync(0xffffffffu, T[m], lane - 3 + a);
+        if (a < 6) vl = a == 0 ? __dmul_rn(kProlongW[5], c) : __dadd_rn(vl, __dmul_rn(kProlongW[5 - a], c));
+        if (a > 0) vr = a == 1 ? __dmul_rn(kProlongW[0], c) : __dadd_rn(vr, __dmul_rn(kProlongW[a - 1], c));
+      }
+      const bool row = ((m & 1) ? yo : ye) && ((m & 2) ? zo : ze);
+      if (row && (wl || wr)) {
+        double* o = dst + amr_idx(D, 2 * cx, 2 * cy + (m & 1), 2 * cz + (m >> 1));
+        if (wl) o[0] = vl;
+        if (wr) o[1] = vr;
       }
     }
   }
@@ -149,47 +157,68 @@ __global__ void k_amr_prolong(const AmrBlock* __restrict__ blocks, const AmrBox*
 // Coarse cells of dst (coarse) from fine src: restrict3
 // (prolongrestrict_cell.f90:2330-2468): fine 2k-2..2k+3 with weights
 // C1 C2 C3 C3 C2 C1, z then y then x.  Writes the current state or the
-// time-interpolated temp.  One thread per (field, coarse cell) unit,
-// field-major within a box, so consecutive threads take consecutive cells.
-__global__ void k_amr_restrict(const AmrBlock* __restrict__ blocks, const AmrBox* __restrict__ boxes,
-                               const int2* __restrict__ tiles, int ntiles, int to_temp, unsigned* status) {
+// time-interpolated temp.
+//
+// A lane takes one fine x column and kRestrictRows coarse rows along y: it
+// reduces the column over z once a fine y row (rows of neighbouring coarse
+// cells share four of their six) and over y; every second lane then forms a
+// coarse cell's x sum from its own and five neighbouring columns by shuffle,
+// in the reference's order.  A thread a cell read 216 values of it, every
+// second one of a line (94 us a call of the 48^3 boxes, 33 us now).  A
+// unit is (field, z row, group of y rows, piece of 14 coarse cells): one warp.
+constexpr int kRestrictCells = 14;   // (32 - 4) / 2 coarse cells a warp
+__global__ void __launch_bounds__(128) k_amr_restrict(const AmrBlock* __restrict__ blocks,
+                                                      const AmrBox* __restrict__ boxes, const int2* __restrict__ tiles,
+                                                      int ntiles, int to_temp, unsigned* status) {
   const double C1 = 3.0 / 2.56e2, C2 = -2.5e1 / 2.56e2, C3 = 7.5e1 / 1.28e2;
+  auto sum6 = [&](double a, double b, double c, double d, double e, double g) {
+    return __dadd_rn(__dadd_rn(__dmul_rn(C1, __dadd_rn(a, g)), __dmul_rn(C2, __dadd_rn(b, e))),
+                     __dmul_rn(C3, __dadd_rn(c, d)));
+  };
+  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int2 tile = tiles[t];
     const AmrBox& bx = boxes[tile.x];
     const AmrBlock& D = blocks[bx.dst];
-    const int np = bx.n[0] * bx.n[1] * bx.n[2];
-    const int uu = tile.y + threadIdx.x;
-    if (uu >= np * D.nf) continue;
-    const int f = uu / np, p = uu - f * np;
-    const int c[3] = {bx.lo[0] + p % bx.n[0], bx.lo[1] + (p / bx.n[0]) % bx.n[1], bx.lo[2] + p / (bx.n[0] * bx.n[1])};
     const AmrBlock& S = blocks[bx.src];
-    const int f0[3] = {2 * c[0] - 2, 2 * c[1] - 2, 2 * c[2] - 2};
-    if (!amr_inside(D, c[0], c[1], c[2]) || !amr_inside(S, f0[0], f0[1], f0[2]) ||
-        !amr_inside(S, f0[0] + 5, f0[1] + 5, f0[2] + 5)) {
-      atomicOr(status, ST_BAD_ARG);
+    const RestrictUnits U(bx);
+    const int uu = tile.y + warp;
+    if (uu >= U.count * D.nf) continue;   // a whole warp
+    const int f = uu / U.count, u = uu - f * U.count;
+    const int c0 = bx.lo[0] + (u % U.nx) * kRestrictCells;             // first coarse cell of the piece
+    const int y0 = bx.lo[1] + ((u / U.nx) % U.ny) * kRestrictRows, z = bx.lo[2] + u / (U.nx * U.ny);
+    const int nc = c0 + kRestrictCells < bx.lo[0] + bx.n[0] ? kRestrictCells : bx.lo[0] + bx.n[0] - c0;
+    const int nr = y0 + kRestrictRows < bx.lo[1] + bx.n[1] ? kRestrictRows : bx.lo[1] + bx.n[1] - y0;
+    if (!amr_inside(D, c0, y0, z) || !amr_inside(D, c0 + nc - 1, y0 + nr - 1, z) ||
+        !amr_inside(S, 2 * c0 - 2, 2 * y0 - 2, 2 * z - 2) ||
+        !amr_inside(S, 2 * (c0 + nc - 1) + 3, 2 * (y0 + nr - 1) + 3, 2 * z + 3)) {
+      if (lane == 0) atomicOr(status, ST_BAD_ARG);
       continue;
     }
     const long long sy = S.ex[0], sz = (long long)S.ex[0] * S.ex[1];
-    const double* q = amr_state(S) + f * S.fs + amr_idx(S, f0[0], f0[1], f0[2]);
-    double tmp1[6];
+    const bool col = lane < 2 * nc + 4;   // this lane's fine column 2 c0 - 2 + lane is read
+    const double* q = amr_state(S) + f * S.fs + amr_idx(S, 2 * c0 - 2 + (col ? lane : 0), 2 * y0 - 2, 2 * z - 2);
+    double w[6];   // z sums of fine y rows 2 y - 2 .. 2 y + 3 of the current coarse row
+    auto zsum = [&](int r) {
+      const double* p = q + r * sy;
+      return sum6(p[0], p[sz], p[2 * sz], p[3 * sz], p[4 * sz], p[5 * sz]);
+    };
 #pragma unroll
-    for (int a = 0; a < 6; ++a) {
-      double t2[6];
+    for (int r = 0; r < 4; ++r) w[r + 2] = zsum(r);
+    double* dst = (to_temp ? D.K : amr_state(D)) + f * D.fs;
 #pragma unroll
-      for (int b = 0; b < 6; ++b) {
-        const double* r = q + a + b * sy;
-        t2[b] = __dadd_rn(__dadd_rn(__dmul_rn(C1, __dadd_rn(r[0], r[5 * sz])), __dmul_rn(C2, __dadd_rn(r[sz], r[4 * sz]))),
-                          __dmul_rn(C3, __dadd_rn(r[2 * sz], r[3 * sz])));
-      }
-      tmp1[a] = __dadd_rn(__dadd_rn(__dmul_rn(C1, __dadd_rn(t2[0], t2[5])), __dmul_rn(C2, __dadd_rn(t2[1], t2[4]))),
-                          __dmul_rn(C3, __dadd_rn(t2[2], t2[3])));
+    for (int y = 0; y < kRestrictRows; ++y) {
+      if (y >= nr) break;   // the same in the whole warp
+#pragma unroll
+      for (int r = 0; r < 4; ++r) w[r] = w[r + 2];
+      w[4] = zsum(2 * y + 4);
+      w[5] = zsum(2 * y + 5);
+      const double T = sum6(w[0], w[1], w[2], w[3], w[4], w[5]);
+      double x[6];
+#pragma unroll
+      for (int a = 0; a < 6; ++a) x[a] = __shfl_sync(0xffffffffu, T, lane + a);
+      if ((lane & 1) == 0 && lane / 2 < nc) dst[amr_idx(D, c0 + lane / 2, y0 + y, z)] = sum6(x[0], x[1], x[2], x[3], x[4], x[5]);
     }
-    const double v = __dadd_rn(__dadd_rn(__dmul_rn(C1, __dadd_rn(tmp1[0], tmp1[5])), __dmul_rn(C2, __dadd_rn(tmp1[1], tmp1[4]))),
-                               __dmul_rn(C3, __dadd_rn(tmp1[2], tmp1[3])));
-    const long long od = (long long)f * D.fs + amr_idx(D, c[0], c[1], c[2]);
-    if (to_temp) D.K[od] = v;
-    else amr_state(D)[od] = v;
   }
 }
 

@@ -24,12 +24,37 @@ struct AmrBox {
   int n[3];
 };
 
-// Fine cells per thread of the prolongation (a run along x from an even
-// index), and the runs that cover x cells [lo0, lo0 + n0) of a box.
-constexpr int kProlongRun = 16;
-__host__ __device__ inline int prolong_runs_x(int lo0, int n0) {
-  return ((lo0 + n0) - (lo0 & ~1) + kProlongRun - 1) / kProlongRun;
-}
+// Work units of the prolongation over a box of fine cells (k_amr_prolong):
+// coarse cells c0 .. with a child in the box, pieces of seg - 6 of them along
+// x on segments of seg lanes, per_warp segments a warp; `count` units a field.
+struct ProlongUnits {
+  int c0[3], nc, seg, per_warp, nx, ny, count;
+  __host__ __device__ explicit ProlongUnits(const AmrBox& b) {
+    int n[3];
+    for (int d = 0; d < 3; ++d) {
+      c0[d] = b.lo[d] >> 1;
+      n[d] = ((b.lo[d] + b.n[d] - 1) >> 1) - c0[d] + 1;
+    }
+    nc = n[0];
+    seg = nc <= 4 ? 10 : (nc <= 10 ? 16 : 32);
+    per_warp = 32 / seg;
+    nx = (nc + seg - 7) / (seg - 6);
+    ny = n[1];
+    count = nx * ny * n[2];
+  }
+};
+
+// Work units of the restriction over a box of coarse cells (k_amr_restrict):
+// pieces of 14 cells along x, kRestrictRows rows along y; `count` units a field.
+constexpr int kRestrictRows = 4;
+struct RestrictUnits {
+  int nx, ny, count;
+  __host__ __device__ explicit RestrictUnits(const AmrBox& b) {
+    nx = (b.n[0] + 13) / 14;
+    ny = (b.n[1] + kRestrictRows - 1) / kRestrictRows;
+    count = nx * ny * b.n[2];
+  }
+};
 
 enum AmrBuf : int { BUF_STATE = 0, BUF_STAGE_A = 1, BUF_STAGE_B = 2, BUF_TEMP = 3 };
 
