@@ -41,7 +41,7 @@ cudaError_t launch_face(const void* blocks, const int2* faces, int nfaces, int s
                         unsigned* status, cudaStream_t s);
 template <typename T, typename SS>
 cudaError_t launch_deriv(const void* blocks, const DerivItem* items, int nitems, int sub, void* D, int slots,
-                         int region, int grid, cudaStream_t s, int occ);
+                         int region, int grid, cudaStream_t s);
 
 // out = E(in) on the metric / A~ fields; other fields copied.
 __global__ void k_enforce_copy(const double* __restrict__ in, double* __restrict__ out, long long n, long long fs) {
@@ -75,8 +75,10 @@ struct amss_adjoint {
   StepBlock<double>* dtab = nullptr;     // 4 tables, one per substep
   AdjBlock host_adj{};
   AdjBlock* dadj = nullptr;
-  DerivItem* ditems = nullptr;
+  DerivItem* ditems = nullptr;          // stencil pass
   int nitems = 0;
+  TgItem* dgitems = nullptr;            // its transpose
+  int ngitems = 0;
   int2* dtiles = nullptr;
   int ntiles = 0;
   int2* dfaces = nullptr;
@@ -156,7 +158,7 @@ int fwd_step(amss_adjoint* a, const double* U0raw, double* Unew, double* Z0, dou
   for (int sub = 0; sub < 4; ++sub) {
     const StepBlock<double>* T = a->dtab + sub;
     double* D = Dsub ? Dsub[sub] : a->D;
-    AMSS_CK((launch_deriv<double, double>(T, a->ditems, a->nitems, sub, D, D_SLOTS, -1, std::min(a->nitems, 148 * 16), s, 0)));
+    AMSS_CK((launch_deriv<double, double>(T, a->ditems, a->nitems, sub, D, D_SLOTS, -1, std::min(a->nitems, 148 * 16), s)));
     AMSS_CK((launch_pointwise<double, double, false>(T, a->dtiles, a->ntiles, sub, rk, 0, a->dstatus, s, D)));
     AMSS_CK((launch_face<double, double>(T, a->dfaces, a->nfaces, sub, rk, 0, a->dstatus, s)));
     a->launches += 3;
@@ -175,7 +177,7 @@ int rhs_vjp(amss_adjoint* a, int sub, const double* Xin, const double* Rbv, doub
   cudaStream_t s = a->stream;
   const StepBlock<double>* T = a->dtab + sub;
   if (!Dpre) {
-    AMSS_CK((launch_deriv<double, double>(T, a->ditems, a->nitems, sub, a->D, D_SLOTS, -1, std::min(a->nitems, 148 * 16), s, 0)));
+    AMSS_CK((launch_deriv<double, double>(T, a->ditems, a->nitems, sub, a->D, D_SLOTS, -1, std::min(a->nitems, 148 * 16), s)));
     a->launches++;
   }
   a->host_adj.D = Dpre ? Dpre : a->D;
@@ -185,7 +187,7 @@ int rhs_vjp(amss_adjoint* a, int sub, const double* Xin, const double* Rbv, doub
   AMSS_CK(cudaMemcpyAsync(a->dadj, &a->host_adj, sizeof(AdjBlock), cudaMemcpyHostToDevice, s));
   k_rhs_vjp<<<dim3(grid_of(a->npts), 1), 128, 0, s>>>(a->dadj, a->Db);
   AMSS_CK(cudaGetLastError());
-  k_stencil_gather_tiled<<<a->nitems, DTHREADS, kTgSmem, s>>>(a->dadj, a->ditems, a->Db);
+  k_stencil_gather_tiled<<<a->ngitems, DTHREADS, kTgSmem, s>>>(a->dadj, a->dgitems, a->Db);
   AMSS_CK(cudaGetLastError());
   k_beta_adjoint<<<grid_of(a->npts), 128, 0, s>>>(a->dadj, a->Db);
   AMSS_CK(cudaGetLastError());
@@ -268,7 +270,6 @@ extern "C" amss_adjoint* amss_adjoint_create(const int ex[3], const double bbox[
   s.npts = a->npts;
   s.lev0 = 1;
   s.nf = NFIELDS_BSSN;
-  s.dw = deriv_tile_w(ex[0]);
   for (int t = 0; t < 4; ++t) a->host_tab[t] = s;
   a->host_adj.b = s.b;
   a->host_adj.C = s.C;
@@ -277,15 +278,26 @@ extern "C" amss_adjoint* amss_adjoint_create(const int ex[3], const double bbox[
   a->host_adj.D = a->D;
   a->host_adj.dfs = a->fs;
 
-  std::vector<DerivItem> items;
+  std::vector<DerivItem> cut, items;
+  std::vector<TgItem> gitems;
   std::vector<int2> tiles, faces;
-  const int tw = deriv_tile_w(ex[0]), th = deriv_tile_h(ex[0]);
   static const int order[24] = {F_CHI, F_LAP, F_BETAX, F_BETAY, F_BETAZ, F_GXX, F_GXY, F_GXZ,
                                 F_GYY, F_GYZ, F_GZZ, F_TRK, F_GAMX, F_GAMY, F_GAMZ, F_AXX,
                                 F_AXY, F_AXZ, F_AYY, F_AYZ, F_AZZ, F_DTSFX, F_DTSFY, F_DTSFZ};
-  for (int f : order)
+  const int lo[3] = {0, 0, 0};
+  deriv_push(cut, 0, lo, ex, DWMAX, 1, kAutoSlab);
+  const int slabs = deriv_slabs(cut, false, 2 * 148);
+  cut.clear();
+  deriv_push(cut, 0, lo, ex, DWMAX, slabs, kAutoSlab);
+  for (int f : order) {
+    for (DerivItem it : cut) {
+      it.field = f;
+      items.push_back(it);
+    }
+    const int tw = tg_tile_w(ex[0]), th = DTHREADS / tw;
     for (int y0 = 0; y0 < ex[1]; y0 += th)
-      for (int x0 = 0; x0 < ex[0]; x0 += tw) items.push_back(DerivItem{0, x0, y0, f});
+      for (int x0 = 0; x0 < ex[0]; x0 += tw) gitems.push_back(TgItem{x0, y0, f});
+  }
   for (long long p = 0; p < a->npts; p += kPointwiseTile) tiles.push_back(make_int2(0, (int)p));
   const int fm = s.b.face_mask;
   for (int k = 0; k < ex[2]; ++k)
@@ -296,13 +308,16 @@ extern "C" amss_adjoint* amss_adjoint_create(const int ex[3], const double bbox[
         if (on) faces.push_back(make_int2(0, (int)(i + (long long)j * ex[0] + (long long)k * ex[0] * ex[1])));
       }
   a->nitems = (int)items.size();
+  a->ngitems = (int)gitems.size();
   a->ntiles = (int)tiles.size();
   a->nfaces = (int)faces.size();
   if (cudaMalloc(&a->ditems, items.size() * sizeof(DerivItem)) != cudaSuccess ||
+      cudaMalloc(&a->dgitems, gitems.size() * sizeof(TgItem)) != cudaSuccess ||
       cudaMalloc(&a->dtiles, tiles.size() * sizeof(int2)) != cudaSuccess ||
       (a->nfaces && cudaMalloc(&a->dfaces, faces.size() * sizeof(int2)) != cudaSuccess))
     return fail("amss_adjoint_create: device allocation failed");
   cudaMemcpy(a->ditems, items.data(), items.size() * sizeof(DerivItem), cudaMemcpyHostToDevice);
+  cudaMemcpy(a->dgitems, gitems.data(), gitems.size() * sizeof(TgItem), cudaMemcpyHostToDevice);
   cudaMemcpy(a->dtiles, tiles.data(), tiles.size() * sizeof(int2), cudaMemcpyHostToDevice);
   if (a->nfaces) cudaMemcpy(a->dfaces, faces.data(), faces.size() * sizeof(int2), cudaMemcpyHostToDevice);
   return a;
@@ -311,7 +326,7 @@ extern "C" amss_adjoint* amss_adjoint_create(const int ex[3], const double bbox[
 extern "C" void amss_adjoint_destroy(amss_adjoint* a) {
   if (!a) return;
   if (a->stream) cudaStreamSynchronize(a->stream);
-  void* ptrs[] = {a->dstatus, a->dlvl, a->dcoord, a->dtab, a->dadj, a->ditems, a->dtiles, a->dfaces, a->D, a->Db,
+  void* ptrs[] = {a->dstatus, a->dlvl, a->dcoord, a->dtab, a->dadj, a->ditems, a->dgitems, a->dtiles, a->dfaces, a->D, a->Db,
                   a->U, a->U0, a->X[0], a->X[1], a->X[2], a->K, a->Zs, a->H, a->dloss, a->seg, a->Ub, a->U0b,
                   a->Rb[0], a->Rb[1], a->Rb[2], a->Rb[3], a->Xb, a->Dseg};
   for (void* p : ptrs)
@@ -345,7 +360,7 @@ static int loss_and_grad(amss_adjoint* a, double* loss, bool want_grad) {
   const int gw = 3;
   a->host_tab[0].tl[0] = a->U;   // stencil pass of U (substep-0 input)
   AMSS_CK(cudaMemcpyAsync(a->dtab, a->host_tab, sizeof(StepBlock<double>), cudaMemcpyHostToDevice, s));
-  AMSS_CK((launch_deriv<double, double>(a->dtab, a->ditems, a->nitems, 0, a->D, D_SLOTS, -1, std::min(a->nitems, 148 * 16), s, 0)));
+  AMSS_CK((launch_deriv<double, double>(a->dtab, a->ditems, a->nitems, 0, a->D, D_SLOTS, -1, std::min(a->nitems, 148 * 16), s)));
   a->host_adj.D = a->D;
   a->host_adj.X = a->U;
   a->host_adj.Rb = nullptr;
@@ -360,7 +375,7 @@ static int loss_and_grad(amss_adjoint* a, double* loss, bool want_grad) {
     AMSS_CK(cudaMemsetAsync(a->Db, 0, (size_t)D_SLOTS * a->fs * sizeof(double), s));
     k_ham_vjp<<<dim3(grid_of(a->npts), 1), 128, 0, s>>>(a->dadj, gw, dV, a->H, a->Db);
     AMSS_CK(cudaGetLastError());
-    k_stencil_gather_tiled<<<a->nitems, DTHREADS, kTgSmem, s>>>(a->dadj, a->ditems, a->Db);   // H reads no adv slot
+    k_stencil_gather_tiled<<<a->ngitems, DTHREADS, kTgSmem, s>>>(a->dadj, a->dgitems, a->Db);   // H reads no adv slot
     AMSS_CK(cudaGetLastError());
     a->launches += 2;
   }

@@ -227,16 +227,27 @@ struct TgMap {
     return 0;
   }
 };
-constexpr int kTgPlane = DPLANE;                       // cells of one staged plane (>= (W+6)(H+6))
+// Its tile is W x H columns, one thread a column: W = the block's x extent cut
+// into pieces of at most 64, H = DTHREADS / W rows.
+struct TgItem {
+  int x0, y0, field;
+};
+constexpr int kTgPlane = 704;                          // cells of one staged plane (>= (W+6)(H+6))
+constexpr int kTgPer = (kTgPlane + DTHREADS - 1) / DTHREADS;   // plane cells a thread stages
+__host__ __device__ constexpr int tg_tile_w(int ex0) { return (ex0 + (ex0 + 63) / 64 - 1) / ((ex0 + 63) / 64); }
+constexpr bool tg_planes_fit(int w) {
+  return w > 64 || ((w + 6) * (DTHREADS / w + 6) <= kTgPlane && tg_planes_fit(w + 1));
+}
+static_assert(tg_planes_fit(kDerivMinEx), "plane buffer too small for a tile shape");
 constexpr size_t kTgSmem = 2 * 10 * kTgPlane * sizeof(double);   // two planes of the widest kind
 
 // The plane cells one thread stages: in-plane offset of each (i + j ex0), or
 // -1 outside the block (zero-filled), fixed for the whole march.
 struct TgCells {
-  int off[DPER];
+  int off[kTgPer];
   __device__ __forceinline__ void init(int x0, int y0, int DSX, int np, int ex0, int ex1) {
 #pragma unroll
-    for (int e = 0; e < DPER; ++e) {
+    for (int e = 0; e < kTgPer; ++e) {
       const int t = threadIdx.x + e * DTHREADS;
       const int i = x0 - 3 + t % DSX, j = y0 - 3 + t / DSX;
       off[e] = (t < np && i >= 0 && i < ex0 && j >= 0 && j < ex1) ? i + j * ex0 : (t < np ? -1 : -2);
@@ -254,7 +265,7 @@ __device__ __forceinline__ void tg_stage(const AdjBlock& A, const double* Db, in
     const double* base =
         (sr >= 0 ? Db + (long long)(s0 + sr) * A.dfs : A.X + (long long)(F_BETAX - 1 - sr) * A.b.fs) + zoff;
 #pragma unroll
-    for (int e = 0; e < DPER; ++e) {
+    for (int e = 0; e < kTgPer; ++e) {
       const int o = cells.off[e];
       if (o >= -1) cp_async8(buf + a * kTgPlane + threadIdx.x + e * DTHREADS, o >= 0 ? base + o : base, o >= 0);
     }
@@ -315,7 +326,7 @@ __device__ __forceinline__ void tg_column(const AdjBlock& A, const double* __res
   const Coef<double>& C = A.C.t;
   const int ex0 = b.ex[0], ex1 = b.ex[1], ex2 = b.ex[2];
   const int hix = ex0 - 1, hiy = ex1 - 1, hiz = ex2 - 1;
-  const int W = deriv_tile_w(ex0), H = DTHREADS / W;
+  const int W = tg_tile_w(ex0), H = DTHREADS / W;
   const int DSX = W + 6, np = DSX * (H + 6);
   const int li = threadIdx.x % W, lj = threadIdx.x / W;
   const int x = x0 + li, y = y0 + lj;
@@ -478,13 +489,12 @@ __device__ __forceinline__ void tg_column(const AdjBlock& A, const double* __res
   cp_async_wait<0>();
 }
 
-// Xb += transpose(stencil pass)(Db), one CTA per (tile, field) item of the
-// stencil pass's work list (BSSN layout, no symmetry planes).
+// Xb += transpose(stencil pass)(Db), one CTA per (tile, field) item (BSSN layout, no symmetry planes).
 __global__ void __launch_bounds__(DTHREADS, 2) k_stencil_gather_tiled(const AdjBlock* __restrict__ A,
-                                                                      const DerivItem* __restrict__ items,
+                                                                      const TgItem* __restrict__ items,
                                                                       const double* __restrict__ Db) {
   extern __shared__ __align__(16) unsigned char tg_smem[];
-  const DerivItem it = items[blockIdx.x];
+  const TgItem it = items[blockIdx.x];
   double* smem = reinterpret_cast<double*>(tg_smem);
   switch (dkind(it.field)) {
     case 0: tg_column<0>(*A, Db, it.field, it.x0, it.y0, smem); break;

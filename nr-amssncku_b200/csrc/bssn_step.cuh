@@ -141,7 +141,6 @@ struct StepBlock {
   long long npts;
   int lev0;           // 1: Sommerfeld rule on the patch faces; 0: freeze them at u0
   int nf;             // evolved fields: 24 (BSSN) or 25 (Z4c, Theta last)
-  int dw;             // stencil-pass tile width (deriv_tile_w of ex[0])
   // regions of region tiles, array indices [rlo, rlo + rn): [0] the final
   // substep's, [1] the block's owned cells (its ghosts are synchronised)
   int rlo[2][3], rn[2][3];

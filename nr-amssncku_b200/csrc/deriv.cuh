@@ -1,92 +1,141 @@
 // deriv.cuh -- the stencil pass of the split RK4 substep.
 //
-// One CTA takes one field of one (x, y) tile of a block (W x H points, one
-// thread per column, W and H per block) and marches through z, over the whole
-// block or over the planes [k0, k1) of one z-slab of it.  The planes k .. k+3 of the
-// tile plus a 3-cell halo sit in a 5-slot shared-memory ring, filled as the
-// reference's padded copy fh of symmetry_bd (fmisc.f90:877-901): cells at
-// negative indices hold the mirrored value times the field's parity, cells
-// past the block end are never read by the gated stencils and hold 0.  The
-// next plane is fetched into registers while the current one is computed,
-// so each plane costs one barrier.  The two-CTA form instead copies planes
-// straight into a 6-slot ring with cp.async, two planes ahead, where the
-// source needs no type conversion.
+// One CTA takes one field of one (x, y) tile of a block and marches through z,
+// over the planes [k0, k1) of a z-slab.  A thread owns two columns, adjacent
+// in y.  Planes of the tile lie in a shared-memory ring with a 3-cell halo,
+// filled as the reference's padded copy fh of symmetry_bd (fmisc.f90:877-901):
+// cells at negative indices hold the mirrored value times the field's parity,
+// cells past the block end are never read by the gated stencils and hold 0.
+// x-, y- and z-lines and the xy cross stencil read the ring.  The mixed
+// derivatives with z are Dz(Dx f) and Dz(Dy f) -- the reference's 16-point
+// cross stencils of fdderivs are exactly these tensor products of its 1-D
+// stencils, so only the rounding of the coefficient product differs -- over
+// register windows of Dx f and Dy f at planes k-4 .. k, and are stored two
+// planes late, so that each is formed once.
 //
-// z-direction work comes from registers: each thread keeps its column
-// f(k-3 .. k+3) and the windows of its x- and y-derivatives Dx f, Dy f at
-// planes k-2 .. k+2 (4th order) and k-1 .. k+1 (2nd order), each computed
-// once, when its plane enters the window.  The mixed
-// derivatives with z are formed as Dz(Dx f) and Dz(Dy f): the reference's
-// 16-point (4-point) cross stencils of fdderivs are exactly these tensor
-// products of its 1-D stencils, so only the rounding of the coefficient
-// product differs.  x- and y-lines and the xy cross stencil read the plane.
+// The pass is bound by instruction issue and latency, not by memory (417 MB in
+// 291 us on 70^3 points; of 10,200 instructions a point 2,100 are FP64), so the
+// layout serves those: two columns a thread share the row differences of the
+// cross stencil, the y-line, and a step's barrier, gates and addresses; the
+// row stride is a constant, so that a stencil's reads differ by immediates;
+// the shift comes through shared memory two planes ahead, the coefficients
+// from shared memory; stencils that do not fit are chosen by selects or, for
+// the 2nd-order ones next to an edge, stored over the 4th-order ones.  One
+// column a thread with a register column and per-stencil branches, 35 x 7
+// tiles and whole-block marches took 359 us (mixed 293 us, 200 us now; a 24^3
+// block 72 us, 20 us now, cut into z-slabs).  A second, fully gated path beside
+// a full-width one, in the same warps, was slower (no room in the instruction
+// cache, warps waiting for each other at the plane's barrier).
+//
+// The planes are copied by cp.async into a ring of nine (k-3 .. k+3 in use, k+4
+// landing, k+5 issued), one barrier a plane.  A source that needs conversion
+// (the mixed form's FP64 state at substep 0) lands in a buffer of its own and
+// is converted by the thread that copied it.
 //
 // Per point the pass stores, for the field's kind (stencil.cuh: dslots):
 // gradient, Hessian, and one "adv" value = upwinded advection
 // (lopsidediff.f90:321-481) + eps/64 * KO line sums (kodiss.f90:190-207).
 // The formulas and gates are those of diff_new.f90:946-1528.
 #pragma once
+#include <vector>
+
 #include "bssn_step.cuh"
 
 namespace amss {
 
-// A tile is W x H columns (W <= DWMAX, W * H <= DTHREADS), chosen per block
-// (deriv_tile) so that narrow blocks do not leave lanes idle: W = the block's
-// x extent split into pieces of at most 64, H = DTHREADS / W rows.
 constexpr int DTHREADS = 256;
-// Resident CTAs of DTHREADS threads the stencil pass is compiled for.  Two
-// forms: occupancy 0, two CTAs (128 registers), and occupancy 1, four CTAs in
-// FP64 / three in FP32 arithmetic (64 / 80 registers; the windows spill a few
-// hundred bytes to L1): more warps to cover the plane loads, at the price of
-// the spills.  Which is faster depends on the level (the autotuner picks).
-constexpr int kDerivMinbLow = 2;
-#ifndef AMSS_DERIV_MINB_F64
-#define AMSS_DERIV_MINB_F64 4
-#endif
-#ifndef AMSS_DERIV_MINB_F32
-#define AMSS_DERIV_MINB_F32 3
-#endif
-#ifndef AMSS_DERIV_ASYNC   // 1: the plane ring is filled by cp.async where no type conversion is needed
-#define AMSS_DERIV_ASYNC 1
-#endif
-#ifndef AMSS_DERIV_PREFETCH   // planes beyond the register fetch whose tile rows are prefetched into L2 (0: none)
-#define AMSS_DERIV_PREFETCH 4
-#endif
-constexpr int DWMAX = 64;
-constexpr int DPLANE = 704;                 // >= (W + 6) (H + 6) for every admissible W
-constexpr int DRING = 5;                    // resident planes: k-1 (being replaced), k .. k+3
-constexpr int DRING_ASYNC = 6;              // cp.async ring: k .. k+3, k+4 landing, k+5 issued
-constexpr int DPER = (DPLANE + DTHREADS - 1) / DTHREADS;   // plane cells per thread
-
-// Tile shape of the stencil pass for a block of x extent ex0.
-__host__ __device__ constexpr int deriv_tile_w(int ex0) {
-  return (ex0 + (ex0 + DWMAX - 1) / DWMAX - 1) / ((ex0 + DWMAX - 1) / DWMAX);
-}
-__host__ __device__ constexpr int deriv_tile_h(int ex0) { return DTHREADS / deriv_tile_w(ex0); }
+constexpr int DWMAX = 38;                   // widest tile
+constexpr int DHMAX = 18;                   // highest tile
+constexpr int DS = DWMAX + 6;               // row stride of a plane in shared memory
+constexpr int DPLANE = DS * (DHMAX + 6);    // a plane's slot in the ring
+constexpr int DRING = 9;                    // planes k-3 .. k+3 in use, k+4 landing, k+5 issued
+constexpr int DBETA = 3;                    // planes of the shift: k in use, k+1 landing, k+2 issued
+constexpr int DPER = 4;                     // plane cells a thread copies (deriv_cells_fit)
+// Shared memory: the ring in the widest arithmetic type, which also covers the
+// FP32 ring and its landing planes, then the shift, then the block's stencil
+// coefficients (in registers they spill, from global memory they are waited
+// for).  Two CTAs an SM.
+constexpr size_t kDerivRing = (size_t)DRING * DPLANE * sizeof(double);
+constexpr size_t kDerivCoef = kDerivRing + (size_t)DBETA * 6 * DTHREADS * sizeof(double);
+constexpr size_t kDerivSmem = kDerivCoef + sizeof(Coef<double>);
+static_assert((size_t)DRING * DPLANE * 4 + 2 * DPER * DTHREADS * sizeof(double) <= kDerivRing, "landing planes");
+static_assert(2 * (kDerivSmem + 1024) <= 228 * 1024, "two CTAs an SM");
 constexpr int kDerivMinEx = 8;              // the split form needs blocks at least this wide in x
-constexpr bool deriv_planes_fit(int w) {
-  return w > DWMAX || ((w + 6) * (DTHREADS / w + 6) <= DPLANE && deriv_planes_fit(w + 1));
-}
-static_assert(deriv_planes_fit(kDerivMinEx), "plane buffer too small for a tile shape");
+constexpr int kPointwiseTile = kDTile;      // points of a tile of the pointwise pass
+constexpr int kMinSlab = 8;                 // fewest planes of a z-slab that is asked for
+constexpr int kAutoSlab = 4;                // and of one that deriv_slabs chooses
+constexpr int kMaxTileW = 64;               // widest tile amss_engine_set_level_tiling takes (used up to DWMAX)
 
-// substep tile of the split form's pointwise pass
-constexpr int kPointwiseTile = kDTile;
-// fewest planes of a z-slab of the stencil pass (each slab pays a 7-plane prologue)
-constexpr int kMinSlab = 8;
+// Tile of a region n0 x n1 columns wide: width w (at most wmax) and height h
+// (even, two rows a thread), cutting the region into near-equal tiles of at
+// most DTHREADS column pairs.
+struct DerivTile { int w, h; };
+__host__ __device__ constexpr DerivTile deriv_tile(int n0, int n1, int wmax) {
+  const int wm = wmax < DWMAX ? wmax : DWMAX;
+  const int nx = (n0 + wm - 1) / wm, w = (n0 + nx - 1) / nx;
+  const int hm = 2 * (DTHREADS / w) < DHMAX ? 2 * (DTHREADS / w) : DHMAX;
+  const int ny = (n1 + hm - 1) / hm;
+  return DerivTile{w, 2 * ((n1 + 2 * ny - 1) / (2 * ny))};
+}
+constexpr bool deriv_cells_fit() {
+  for (int w = 1; w <= DWMAX; ++w) {
+    const int hm = 2 * (DTHREADS / w) < DHMAX ? 2 * (DTHREADS / w) : DHMAX;
+    if ((w + 6) * (hm + 6) > DPER * DTHREADS || w * (hm / 2) > DTHREADS) return false;
+  }
+  return true;
+}
+static_assert(deriv_cells_fit(), "a tile has more cells or columns than its threads take");
 
 struct DerivItem {
-  int block;   // index into the level's StepBlock table
-  int x0, y0;  // tile origin (array indices)
+  int block;           // index into the level's StepBlock table
+  int x0, y0;          // tile origin (array indices)
   int field;
-  int k0 = 0, k1 = 0;   // planes [k0, k1) of the march; k1 == 0: the whole block
-  int x1 = 0, y1 = 0;   // columns x < x1, y < y1 only; 0: up to the block's extent
-  int w = 0;            // tile width; 0: the block's (StepBlock::dw)
+  int k0, k1;          // planes [k0, k1)
+  int x1, y1;          // columns x < x1, y < y1 only
+  int w, h;            // tile
 };
+
+// Appends the work items (of field 0) of a block's region [lo, lo + n): tiles
+// at most wmax wide, `slabs` z-slabs of near-equal height (at least `least`).
+inline void deriv_push(std::vector<DerivItem>& v, int block, const int lo[3], const int n[3], int wmax, int slabs,
+                       int least) {
+  const DerivTile t = deriv_tile(n[0], n[1], wmax);
+  const int most = n[2] / least, ns = slabs < 1 || most < 1 ? 1 : slabs < most ? slabs : most;
+  for (int z = 0; z < ns; ++z) {
+    const int k0 = lo[2] + (int)((long long)n[2] * z / ns), k1 = lo[2] + (int)((long long)n[2] * (z + 1) / ns);
+    for (int y0 = lo[1]; y0 < lo[1] + n[1]; y0 += t.h)
+      for (int x0 = lo[0]; x0 < lo[0] + n[0]; x0 += t.w)
+        v.push_back(DerivItem{block, x0, y0, 0, k0, k1, lo[0] + n[0], lo[1] + n[1], t.w, t.h});
+  }
+}
+// z-slabs of a level whose tiling nobody set, from its items at one slab a
+// block: the number with the least expected time on `ctas` resident CTAs.  An
+// item of p planes takes p + 6 steps (four of warm-up, the prologue about two)
+// of relative cost 1, 0.65 or 0.5 by its field's kind; the launch takes the
+// longest item, or all items shared out plus part of a last one.  A 24^3 block
+// is 48 items of 30 steps uncut and 288 of 10 in six slabs (a step 512 and
+// 243 us); 70^3
+// points are best in two (2.01 ms a step; 2.33 uncut, 2.07 in three).
+inline int deriv_slabs(const std::vector<DerivItem>& one, bool z4c, int ctas) {
+  const double per_tile = 11.0 + (z4c ? 5 : 4) * 0.65 + 9 * 0.5;
+  int best = 1;
+  double least = 0.0;
+  for (int ns = 1; ns <= 16; ++ns) {
+    double sum = 0.0, longest = 0.0;
+    for (const DerivItem& it : one) {
+      const int p = it.k1 - it.k0, most = p / kAutoSlab, n = most < 1 ? 1 : ns < most ? ns : most;
+      const double steps = (p + n - 1) / n + 6;
+      sum += n * steps;
+      if (steps > longest) longest = steps;
+    }
+    const double shared = sum * per_tile / ctas + 0.25 * longest, t = shared > longest ? shared : longest;
+    if (ns == 1 || t < least) { least = t; best = ns; }
+  }
+  return best;
+}
 
 // kind of a field's stencil record: 0 gradient + Hessian + adv, 1 gradient + adv, 2 adv
 __host__ __device__ constexpr int dkind(int F) { return dslots(F) == 10 ? 0 : (dslots(F) == 4 ? 1 : 2); }
-
-__device__ __forceinline__ int ring_slot(int m) { return (m + 3) % DRING; }   // m >= -3
 
 // Asynchronous copies global -> shared of one 8- or 4-byte cell (zero-filled
 // when !valid; the source address is then not read).
@@ -108,418 +157,410 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // pass: the store is marked evict-first (st.global.cs) and leaves L2 to the
 // fields the stencil pass re-reads.
 template <typename T>
-__device__ __forceinline__ void dstore(T* a, T v) {
-  __stcs(a, v);
-}
+__device__ __forceinline__ void dstore(T* a, T v) { __stcs(a, v); }
 
-// The plane cells one thread fills, with their in-plane offsets and the x/y
-// mirror signs, fixed for the whole march.
+// The plane cells one thread copies, fixed for the whole march.  A: type in
+// the ring, S: type of the source.
 template <typename A, typename S>
-struct PlaneFetch {
+struct PlaneCells {
   const S* src;
   long long sz;
   int ex2;
-  int off[DPER];     // i + j * ex0 of the (mirrored) cell, -1: none / past the end
+  int off[DPER];     // i + j * ex0 of the (mirrored) cell; -1: past the block's end, -2: no cell
+  int pos[DPER];     // its place in a ring slot
   unsigned neg;      // bit e: x/y mirroring flips the sign of cell e
-  bool zodd;         // field parity in z is odd
-  A v[DPER];
+  int odd;           // bit d: the field's parity in direction d is odd
 
-  __device__ __forceinline__ void init(const S* s, int F, const int* ex, int x0, int y0, int sx, int np) {
+  __device__ __forceinline__ void init(const S* s, int F, const int* ex, int x0, int y0, int w, int h) {
     src = s;
     sz = (long long)ex[0] * ex[1];
     ex2 = ex[2];
-    zodd = soa_sign(F, 2) < 0;
+    odd = (soa_sign(F, 0) < 0 ? 1 : 0) | (soa_sign(F, 1) < 0 ? 2 : 0) | (soa_sign(F, 2) < 0 ? 4 : 0);
     neg = 0;
+    const int sx = w + 6, np = sx * (h + 6);
 #pragma unroll
     for (int e = 0; e < DPER; ++e) {
       const int t = threadIdx.x + e * DTHREADS;
-      int o = -1;
+      const int cj = t / sx, ci = t - cj * sx;
+      off[e] = -2;
+      pos[e] = 0;
       if (t < np) {
-        int i = x0 - 3 + t % sx, j = y0 - 3 + t / sx;
-        bool n = false;
-        if (i < 0) { i = -i - 1; n ^= soa_sign(F, 0) < 0; }
-        if (j < 0) { j = -j - 1; n ^= soa_sign(F, 1) < 0; }
-        if (i < ex[0] && j < ex[1]) o = i + j * ex[0];
-        if (n) neg |= 1u << e;
-      }
-      off[e] = o;
-    }
-  }
-  // issue the loads of plane kk (negative: mirrored, past the end: 0) into w
-  __device__ __forceinline__ void fetch_to(int kk, A* w) const {
-    int k = kk;
-    bool nz = false;
-    if (k < 0) { k = -k - 1; nz = zodd; }
-    const bool kin = k < ex2;
-#pragma unroll
-    for (int e = 0; e < DPER; ++e) {
-      A x = A(0);
-      if (kin && off[e] >= 0) {
-        x = (A)__ldg(src + off[e] + k * sz);
-        if ((((neg >> e) & 1u) != 0) != nz) x = -x;
-      }
-      w[e] = x;
-    }
-  }
-  __device__ __forceinline__ void fetch(int kk) { fetch_to(kk, v); }
-  __device__ __forceinline__ void store_from(A* slot, int np, const A* w) const {
-#pragma unroll
-    for (int e = 0; e < DPER; ++e) {
-      const int t = threadIdx.x + e * DTHREADS;
-      if (t < np) slot[t] = w[e];
-    }
-  }
-  __device__ __forceinline__ void store(A* slot, int np) const { store_from(slot, np, v); }
-};
-
-// The same plane cells copied straight into the ring by cp.async when the
-// source type is the arithmetic type: no registers hold the plane in flight.
-// Cells past the block end are zero-filled by the copy; a mirrored cell is
-// negated after its copy lands, by the thread that issued it.
-template <typename A>
-struct PlaneAsync {
-  const A* src;
-  long long sz;
-  int ex2, np;
-  int off[DPER];     // i + j * ex0 of the (mirrored) cell, -1: none / past the end
-  unsigned neg;      // bit e: x/y mirroring flips the sign of cell e
-  bool zodd;         // field parity in z is odd
-
-  __device__ __forceinline__ void init(const A* s, int F, const int* ex, int x0, int y0, int sx, int n) {
-    src = s;
-    sz = (long long)ex[0] * ex[1];
-    ex2 = ex[2];
-    np = n;
-    zodd = soa_sign(F, 2) < 0;
-    neg = 0;
-#pragma unroll
-    for (int e = 0; e < DPER; ++e) {
-      const int t = threadIdx.x + e * DTHREADS;
-      int o = -1;
-      if (t < n) {
-        int i = x0 - 3 + t % sx, j = y0 - 3 + t / sx;
+        int i = x0 - 3 + ci, j = y0 - 3 + cj;
         bool m = false;
-        if (i < 0) { i = -i - 1; m ^= soa_sign(F, 0) < 0; }
-        if (j < 0) { j = -j - 1; m ^= soa_sign(F, 1) < 0; }
-        if (i < ex[0] && j < ex[1]) o = i + j * ex[0];
+        if (i < 0) { i = -i - 1; m ^= (odd & 1) != 0; }
+        if (j < 0) { j = -j - 1; m ^= (odd & 2) != 0; }
+        off[e] = i < ex[0] && j < ex[1] ? i + j * ex[0] : -1;
+        pos[e] = cj * DS + ci;
         if (m) neg |= 1u << e;
       }
-      off[e] = o;
     }
   }
-  // issue the copies of plane kk (negative: mirrored, past the end: 0) into slot
-  __device__ __forceinline__ void issue(int kk, A* slot) const {
+  // whether cell e of plane kk takes the opposite sign of its source
+  __device__ __forceinline__ bool flips(int e, int kk) const { return (((neg >> e) & 1u) != 0) != (kk < 0 && (odd & 4)); }
+  // issues the copies of plane kk (negative: mirrored, past the end: 0): into
+  // the ring slot (no conversion), or into buf, one cell per thread and e
+  __device__ __forceinline__ void issue(int kk, A* slot, S* buf) const {
     const int k = kk < 0 ? -kk - 1 : kk;
     const bool kin = k < ex2;
+    const S* pl = src + (kin ? k * sz : 0);
 #pragma unroll
-    for (int e = 0; e < DPER; ++e) {
-      const int t = threadIdx.x + e * DTHREADS;
-      if (t < np) {
+    for (int e = 0; e < DPER; ++e)
+      if (off[e] >= -1) {
         const bool ok = kin && off[e] >= 0;
-        const A* g = ok ? src + off[e] + k * sz : src;
-        if constexpr (sizeof(A) == 8) cp_async8(slot + t, g, ok);
-        else cp_async4(slot + t, g, ok);
+        const S* g = ok ? pl + off[e] : src;
+        void* d = sizeof(A) == sizeof(S) ? (void*)(slot + pos[e]) : (void*)(buf + threadIdx.x + e * DTHREADS);
+        if constexpr (sizeof(S) == 8) cp_async8(d, g, ok);
+        else cp_async4(d, g, ok);
       }
-    }
   }
-  // after the copies of plane kk landed: the signs of its mirrored cells
-  __device__ __forceinline__ void fix(int kk, A* slot) const {
-    const bool nz = kk < 0 && zodd;
-    if (!neg && !nz) return;
-    const int k = kk < 0 ? -kk - 1 : kk;
-    if (k >= ex2) return;
+  // once this thread's copies of plane kk landed: their signs, and the conversion
+  __device__ __forceinline__ void land(int kk, A* slot, const S* buf) const {
+    if constexpr (sizeof(A) == sizeof(S)) {
+      if (!neg && !(kk < 0 && (odd & 4))) return;
 #pragma unroll
-    for (int e = 0; e < DPER; ++e) {
-      const int t = threadIdx.x + e * DTHREADS;
-      if (t < np && off[e] >= 0 && (((neg >> e) & 1u) != 0) != nz) slot[t] = -slot[t];
+      for (int e = 0; e < DPER; ++e)
+        if (off[e] >= 0 && flips(e, kk)) slot[pos[e]] = -slot[pos[e]];
+    } else {
+#pragma unroll
+      for (int e = 0; e < DPER; ++e)
+        if (off[e] >= -1) {
+          const A v = (A)buf[threadIdx.x + e * DTHREADS];
+          slot[pos[e]] = flips(e, kk) ? -v : v;
+        }
     }
   }
 };
 
 // Upwinded term of one direction (lopsidediff.f90:321-481) over a line f(o),
 // o = -3 .. 3 relative to the point; f already includes the +1 of the
-// diagonal metric.  bd = beta * d12.
+// diagonal metric.  bd = beta * d12.  Which stencil a point takes depends on
+// the sign of beta and on the room towards the ends of the line: 0 forward, 1
+// centred, 2 backward -- the forward arithmetic on the mirrored line --, 3
+// none; lop_codes packs the form for beta > 0 (bits 0, 1) and < 0 (bits 2, 3).
+__device__ __forceinline__ int lop_codes(int idx, int lo, int hi) {
+  const int p = idx + 3 <= hi ? 0 : (idx + 2 <= hi ? 1 : (idx + 1 <= hi ? 2 : 3));
+  const int n = idx - 3 >= lo ? 2 : (idx - 2 >= lo ? 1 : (idx - 1 >= lo ? 0 : 3));
+  return p | (n << 2);
+}
 template <typename A, typename FN>
-__device__ __forceinline__ A lop_term(const FN& f, A b, A bd, int idx, int lo, int hi) {
-  const A F3 = A(3), F10 = A(10), F18 = A(18), F6 = A(6), EIT = A(8);
-  if (idx - 3 >= lo && idx + 3 <= hi) {
-    // both full-width branches fit: the same arithmetic on the mirrored line,
-    // chosen by selects instead of divergent branches
-    const bool pos = b > A(0);
-    const A fa = pos ? f(-1) : f(1), fb = f(0), fc = pos ? f(1) : f(-1);
-    const A fd = pos ? f(2) : f(-2), fe = pos ? f(3) : f(-3);
-    const A s = -F3 * fa - F10 * fb + F18 * fc - F6 * fd + fe;
-    return pos ? bd * s : (b < A(0) ? -bd * s : A(0));
+__device__ __forceinline__ A lop_term(const FN& f, A b, A bd, int codes) {
+  const int form = b > A(0) ? (codes & 3) : (b < A(0) ? codes >> 2 : 3);
+  const bool fwd = form == 0;
+  const A F3 = A(3), F10 = A(10), F18 = A(18), F6 = A(6);
+  const A fa = fwd ? f(-1) : f(1), fb = f(0), fc = fwd ? f(1) : f(-1);
+  const A fd = fwd ? f(2) : f(-2), fe = fwd ? f(3) : f(-3);
+  const A s = -F3 * fa - F10 * fb + F18 * fc - F6 * fd + fe;
+  A r = (fwd ? bd : -bd) * s;
+  if (form & 1) r = form == 1 ? bd * (f(-2) - A(8) * f(-1) + A(8) * f(1) - f(2)) : A(0);
+  return r;
+}
+
+// KO dissipation of a point from its three lines, each taken with `add` added
+// (Z4C: 1 for the diagonal metric, Z4c_rhs.f90:1240-1245; BSSN adds nothing).
+template <typename A, bool Z4C, typename FX, typename FY, typename FZ>
+__device__ __forceinline__ A ko_term(const FX& X, const FY& Y, const FZ& Z, A add, const Coef<A>& C) {
+  if constexpr (Z4C && sizeof(A) == 8) {
+    auto x = [&](int o) { return __dadd_rn(X(o), add); };
+    auto y = [&](int o) { return __dadd_rn(Y(o), add); };
+    auto z = [&](int o) { return __dadd_rn(Z(o), add); };
+    return kodiv(ko_sum_rn<A, false>(x), C, 0) + kodiv(ko_sum_rn<A, false>(y), C, 1) + kodiv(ko_sum_rn<A, false>(z), C, 2);
+  } else {
+    return kodiv(ko_sum_rn<A, false>(X), C, 0) + kodiv(ko_sum_rn<A, false>(Y), C, 1) + kodiv(ko_sum_rn<A, false>(Z), C, 2);
   }
-  A d = A(0);
-  if (b > A(0)) {
-    if (idx + 3 <= hi) d = bd * (-F3 * f(-1) - F10 * f(0) + F18 * f(1) - F6 * f(2) + f(3));
-    else if (idx + 2 <= hi) d = bd * (f(-2) - EIT * f(-1) + EIT * f(1) - f(2));
-    else if (idx + 1 <= hi) d = -bd * (-F3 * f(1) - F10 * f(0) + F18 * f(-1) - F6 * f(-2) + f(-3));
-  } else if (b < A(0)) {
-    if (idx - 3 >= lo) d = -bd * (-F3 * f(1) - F10 * f(0) + F18 * f(-1) - F6 * f(-2) + f(-3));
-    else if (idx - 2 >= lo) d = bd * (f(-2) - EIT * f(-1) + EIT * f(1) - f(2));
-    else if (idx - 1 >= lo) d = bd * (-F3 * f(-1) - F10 * f(0) + F18 * f(1) - F6 * f(2) + f(3));
-  }
-  return d;
 }
 
 // March one field of one tile.  A: stencil arithmetic type, S: type of the
 // field's source array, SI: type of the stage input (for the shift), T: type
 // of the D array.
-template <typename A, int KIND, bool ASYNC, typename T, typename S, typename SI>
-__device__ __forceinline__ void deriv_column(const StepBlock<T>& B, const S* src, const SI* in, const double* bsh,
-                                             int F, const DerivItem& it, T* D, int slots, int region, A* ring) {
-  const Coef<A>& C = pick<A>(B.C);
+template <typename A, int KIND, bool Z4C, typename T, typename S, typename SI>
+__device__ __forceinline__ void deriv_march(const StepBlock<T>& B, const S* src, const SI* in, const double* bsh,
+                                            int F, const DerivItem& it, T* D, int slots, int region,
+                                            unsigned char* smem) {
+  const Coef<A>& C = *reinterpret_cast<const Coef<A>*>(smem + kDerivCoef);
+  if (threadIdx.x < sizeof(Coef<A>) / 4)
+    reinterpret_cast<unsigned*>(smem + kDerivCoef)[threadIdx.x] = reinterpret_cast<const unsigned*>(&pick<A>(B.C))[threadIdx.x];
+  A* ring = reinterpret_cast<A*>(smem);
+  S* land = reinterpret_cast<S*>(smem + (size_t)DRING * DPLANE * sizeof(A));   // two planes, where A != S
+  // the thread's shift values, component c of point a of plane k at
+  // ((k % DBETA) * 6 + 2 c + a) * DTHREADS
+  double* bet = reinterpret_cast<double*>(smem + kDerivRing) + threadIdx.x;
   const int ex0 = B.b.ex[0], ex1 = B.b.ex[1], ex2 = B.b.ex[2];
-  const int x0 = it.x0, y0 = it.y0, k0 = it.k0;
-  const int kend = it.k1 > 0 ? it.k1 : ex2;
-  const int xend = it.x1 > 0 ? it.x1 : ex0, yend = it.y1 > 0 ? it.y1 : ex1;
+  const int x0 = it.x0, y0 = it.y0, k0 = it.k0, k1 = it.k1, W = it.w, NP = it.h / 2;
   const long long fs = B.b.fs;
-  const int W = it.w > 0 ? it.w : B.dw, H = DTHREADS / W;
-  const int DSX = W + 6;                     // row stride of the plane buffer
-  const int np = DSX * (H + 6);              // cells of one plane (<= DPLANE)
-  const int li = threadIdx.x % W, lj = threadIdx.x / W;
-  const int i = x0 + li, j = y0 + lj;
-  const bool mine = lj < H && i < xend && j < yend;
-  const int fm = B.b.face_mask;
-  const bool face_xy = ((fm & 1) && i == ex0 - 1) || ((fm & 2) && j == ex1 - 1) || ((fm & 8) && i == 0) ||
-                       ((fm & 16) && j == 0);
+  const int fm = B.b.face_mask, ls = B.b.lowsym_mask;
+  const int lox = (ls & 1) ? -3 : 0, loy = (ls & 2) ? -3 : 0, loz = (ls & 4) ? -3 : 0;
+
+  // The thread's column pair (li, 2 pj), (li, 2 pj + 1) of the tile, row by row.
+  const int pj = threadIdx.x / W, li = threadIdx.x - pj * W;
+  const bool any = pj < NP;
+  const int i = x0 + li, j = y0 + 2 * pj;
+  const bool xin = any && i < it.x1 && !((fm & 1) && i == ex0 - 1) && !((fm & 8) && i == 0);
+  const bool m0 = xin && j < it.y1 && !((fm & 2) && j == ex1 - 1) && !((fm & 16) && j == 0);
+  const bool m1 = xin && j + 1 < it.y1 && !((fm & 2) && j + 1 == ex1 - 1);
+  const int own = any ? (2 * pj + 3) * DS + li + 3 : 0;   // in a ring slot
+  // which stencils fit in x and y at the two points (the z part is the plane's):
+  // bit 0 4th order, 1 2nd order, 2 KO, 3 advection (point_gates)
+  auto fits_xy = [&](int jj) -> int {
+    const int lx = (ls & 1) ? -2 : 0, ly = (ls & 2) ? -2 : 0;
+    const int nx = i - lx < ex0 - 1 - i ? i - lx : ex0 - 1 - i, ny = jj - ly < ex1 - 1 - jj ? jj - ly : ex1 - 1 - jj;
+    const int n = nx < ny ? nx : ny;   // cells to the nearest end, mirrored ones (two of them) included
+    const int mx = i - lox < ex0 - 1 - i ? i - lox : ex0 - 1 - i, my = jj - loy < ex1 - 1 - jj ? jj - loy : ex1 - 1 - jj;
+    return (n >= 2 ? 1 : 0) | (n >= 1 ? 2 : 0) | ((mx < my ? mx : my) >= 3 ? 4 : 0) |
+           (i <= ex0 - 2 && jj <= ex1 - 2 ? 8 : 0);
+  };
+  const int fit0 = fits_xy(j), fit1 = fits_xy(j + 1);
+  auto fits_z = [&](int k) -> int {
+    const int lz = (ls & 4) ? -2 : 0, n = k - lz < ex2 - 1 - k ? k - lz : ex2 - 1 - k;
+    return (n >= 2 ? 1 : 0) | (n >= 1 ? 2 : 0) | (k - 3 >= loz && k + 3 < ex2 ? 4 : 0) | (k <= ex2 - 2 ? 8 : 0);
+  };
+
+  // entries of the points in their tiles' order, and the D rows of the field
+  const int rn0 = region < 0 ? ex0 : B.rn[region][0], rn1 = region < 0 ? ex1 : B.rn[region][1];
+  const int rx = region < 0 ? 0 : B.rlo[region][0], ry = region < 0 ? 0 : B.rlo[region][1];
+  const int rz = region < 0 ? 0 : B.rlo[region][2];
+  const int og = dl::g(F) * kDTile, oh = dl::h(F) * kDTile, oa = dl::a(F) * kDTile;
+  auto dptr = [&](int a, int k) -> T* {
+    const int dq = (i - rx) + rn0 * ((j + a - ry) + rn1 * (k - rz));
+    return D + ((long long)(B.dtile + (dq >> 7)) * (slots * kDTile) + (dq & 127));
+  };
+  static_assert(kDTile == 128, "dptr");
+
   // the diagonal metric is advected as g = d + 1 (bssn_rhs.f90:948-953) in FP64,
   // bit-faithful to the reference; FP32 advects d (the constant drops out)
   const A add1 = (sizeof(A) == 8 && (F == F_GXX || F == F_GYY || F == F_GZZ)) ? A(1) : A(0);
-  // D rows of the field's terms, and the point's entry in its tile order
-  const int og = dl::g(F) * kDTile, oh = dl::h(F) * kDTile, oa = dl::a(F) * kDTile;
-  const int rx = region < 0 ? 0 : B.rlo[region][0], ry = region < 0 ? 0 : B.rlo[region][1];
-  const int rz = region < 0 ? 0 : B.rlo[region][2];
-  const int rn0 = region < 0 ? ex0 : B.rn[region][0], rn1 = region < 0 ? ex1 : B.rn[region][1];
-  const int own = (lj < H ? lj + 3 : 3) * DSX + (li + 3);   // idle threads read a valid cell
 
-  // ASYNC: cp.async fills the ring where the source needs no conversion (six
-  // slots: planes k .. k+3 read, k+4 landing, k+5 issued); otherwise the
-  // planes pass through registers (five slots)
-  constexpr bool kAsync = ASYNC && sizeof(A) == sizeof(S);
-  constexpr int R = kAsync ? DRING_ASYNC : DRING;
-  auto rs = [](int m) { return (m + 3) % R; };   // ring slot of plane m >= -3
-  PlaneFetch<A, S> P;
-  PlaneAsync<A> PA;
-  if constexpr (kAsync) PA.init(reinterpret_cast<const A*>(src), F, B.b.ex, x0, y0, DSX, np);
-  else P.init(src, F, B.b.ex, x0, y0, DSX, np);
+  PlaneCells<A, S> P;
+  P.init(src, F, B.b.ex, x0, y0, W, it.h);
 
-  A c[7];                  // column f(k-3 .. k+3)
-  A fx4[5], fy4[5];        // 4th-order Dx f, Dy f at planes k-2 .. k+2 (KIND 0)
-  A fx2[3], fy2[3];        // 2nd-order Dx f, Dy f at planes k-1 .. k+1 (KIND 0)
+  A wx0[5], wy0[5];        // Dx f, Dy f at planes k-4 .. k (KIND 0)
+  A wx1[5], wy1[5];
+#pragma unroll
+  for (int t = 0; t < 5; ++t) wx0[t] = wy0[t] = wx1[t] = wy1[t] = A(0);
 
-  auto dx4 = [&](const A* q) { return C.d12[0] * (q[-2] - A(8) * q[-1] + A(8) * q[1] - q[2]); };
-  auto dy4 = [&](const A* q) { return C.d12[1] * (q[-2 * DSX] - A(8) * q[-DSX] + A(8) * q[DSX] - q[2 * DSX]); };
-  auto dx2 = [&](const A* q) { return C.d2[0] * (-q[-1] + q[1]); };
-  auto dy2 = [&](const A* q) { return C.d2[1] * (-q[-DSX] + q[DSX]); };
-
-  // prologue: the column gets planes k0-3 .. k0+3 and the derivative windows
-  // planes k0-2 .. k0+1.  Register form: the loads of the seven planes are
-  // issued together, then the planes enter the ring one at a time.  cp.async
-  // form: planes k0-3 .. k0+2 fill the six slots at once; once they are read,
-  // k0+3 and k0+4 take the slots of k0-3 and k0-2.
-  A pro[kAsync ? 1 : 7][DPER];
-  if constexpr (kAsync) {
+  // the shift at the points of plane k, from the stage input (bsh: its FP64
+  // side slots in the mixed form), copied two planes ahead
+  auto shift = [&](int k) {
+    if (k < k0 || k >= k1) return;
+    const double* b = sizeof(SI) == 4 ? bsh : (const double*)in + F_BETAX * fs;
+    const double* g = b + i + (long long)j * ex0 + (long long)k * P.sz;
+    double* s = bet + (k % DBETA) * 6 * DTHREADS;
 #pragma unroll
-    for (int m = -3; m <= 2; ++m) PA.issue(k0 + m, ring + rs(k0 + m) * DPLANE);
-    cp_async_commit();
-    cp_async_wait<0>();
-#pragma unroll
-    for (int m = -3; m <= 2; ++m) PA.fix(k0 + m, ring + rs(k0 + m) * DPLANE);
-    __syncthreads();
-  } else {
-#pragma unroll
-    for (int m = -3; m <= 3; ++m) P.fetch_to(k0 + m, pro[m + 3]);
-  }
-#pragma unroll
-  for (int m = -3; m <= 3; ++m) {
-    A* slot = ring + rs(k0 + m) * DPLANE;
-    if constexpr (kAsync) {
-      if (m == 3) {
-        __syncthreads();   // planes k0-3, k0-2 are read: their slots take k0+3, k0+4
-        PA.issue(k0 + 3, slot);
-        cp_async_commit();
-        PA.issue(k0 + 4, ring + rs(k0 + 4) * DPLANE);
-        cp_async_commit();
-        cp_async_wait<1>();
-        PA.fix(k0 + 3, slot);
-        __syncthreads();
-      }
-    } else {
-      P.store_from(slot, np, pro[m + 3]);
-      __syncthreads();
+    for (int c = 0; c < 3; ++c) {
+      if (m0) cp_async8(s + 2 * c * DTHREADS, g + c * fs, true);
+      if (m1) cp_async8(s + (2 * c + 1) * DTHREADS, g + c * fs + ex0, true);
     }
-    const A* q = slot + own;
-    const A cm = q[0];
-#pragma unroll
-    for (int t = 0; t < 7; ++t)
-      if (t == m + 3) c[t] = cm;
-    if constexpr (KIND == 0) {
-      if (m >= -2 && m <= 1) {
-        const A a4 = dx4(q), b4 = dy4(q), a2 = dx2(q), b2 = dy2(q);
-#pragma unroll
-        for (int t = 0; t < 4; ++t)
-          if (t == m + 2) { fx4[t] = a4; fy4[t] = b4; }
-#pragma unroll
-        for (int t = 0; t < 2; ++t)
-          if (t == m + 1) { fx2[t] = a2; fy2[t] = b2; }
-      }
-    }
-  }
+  };
 
+  // Planes kA-1 .. kA+4, kA = k0 - 2, fill six slots of the ring: plane m in
+  // slot (m - kA) mod DRING.  (Planes kA-3, kA-2 are read by no point.)
+  const int kA = k0 - 2;
+  auto first = [&](int m) { return ring + (m < 0 ? DRING - 1 : m) * DPLANE; };
+  if constexpr (sizeof(A) == sizeof(S)) {
 #pragma unroll 1
-  for (int k = k0; k < kend; ++k) {
-    // in flight while plane k is computed: plane k+4 (registers) or k+5 (cp.async)
-    if constexpr (kAsync) {
-      PA.issue(k + 5, ring + rs(k + 5) * DPLANE);
+    for (int m = -1; m <= 4; ++m) {
+      P.issue(kA + m, first(m), land);
+      if (m >= 3) cp_async_commit();
+    }
+    cp_async_wait<1>();
+#pragma unroll 1
+    for (int m = -1; m <= 3; ++m) P.land(kA + m, first(m), land);
+  } else {
+    // one plane after another through the landing buffer
+#pragma unroll 1
+    for (int m = -1; m <= 3; ++m) {
+      P.issue(kA + m, nullptr, land + (m & 1) * (DPER * DTHREADS));
       cp_async_commit();
-    } else {
-      P.fetch(k + 4);
-    }
-#if AMSS_DERIV_PREFETCH
-    {
-      // warp 0 asks L2 for the tile rows (with halo) of plane k+4+AMSS_DERIV_PREFETCH,
-      // one 128-byte line per lane, so the register fetch of that plane meets L2
-      const int kk = k + 4 + AMSS_DERIV_PREFETCH;
-      if (threadIdx.x < 32 && kk < ex2 && kk < kend + 3) {
-        const int xl = x0 - 3 < 0 ? 0 : x0 - 3, xh = x0 + W + 3 > ex0 ? ex0 : x0 + W + 3;
-        const int yl = y0 - 3 < 0 ? 0 : y0 - 3, yh = y0 + H + 3 > ex1 ? ex1 : y0 + H + 3;
-        const int lpr = (int)(((xh - xl) * sizeof(S) + 127) / 128);   // lines per row
-        for (int t = threadIdx.x; t < lpr * (yh - yl); t += 32) {
-          const int r = t / lpr, c = t - r * lpr;
-          const char* row = (const char*)(src + xl + (long long)(yl + r) * ex0 + (long long)kk * ex0 * ex1);
-          const long long off = (long long)c * 128 < (long long)((xh - xl - 1) * sizeof(S)) ? (long long)c * 128
-                                                                                           : (long long)((xh - xl - 1) * sizeof(S));
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(row + off));
-        }
+      if (m >= 0) {
+        cp_async_wait<1>();
+        P.land(kA + m - 1, first(m - 1), land + ((m - 1) & 1) * (DPER * DTHREADS));
       }
     }
-#endif
-    const A* qk = ring + rs(k) * DPLANE + own;
-    c[6] = ring[rs(k + 3) * DPLANE + own];
-    if constexpr (KIND == 0) {
-      const A* q2 = ring + rs(k + 2) * DPLANE + own;
-      const A* q1 = ring + rs(k + 1) * DPLANE + own;
-      fx4[4] = dx4(q2); fy4[4] = dy4(q2); fx2[2] = dx2(q1); fy2[2] = dy2(q1);
-    }
-    const bool on_face = face_xy || ((fm & 4) && k == ex2 - 1) || ((fm & 32) && k == 0);
-    if (mine && !on_face) {
-      const PointGates G = point_gates(B.b, i, j, k);
-      const long long p = i + (long long)j * ex0 + (long long)k * ex0 * ex1;
-      const long long dq = (i - rx) + (long long)rn0 * ((j - ry) + (long long)rn1 * (k - rz));
-      T* d = D + (B.dtile + dq / kDTile) * ((long long)slots * kDTile) + dq % kDTile;
-      auto X = [&](int dd) { return qk[dd]; };
-      auto Y = [&](int dd) { return qk[dd * DSX]; };
-      auto Z = [&](int dd) { return c[3 + dd]; };
-      if constexpr (KIND <= 1) {
-        A gx = A(0), gy = A(0), gz = A(0);
-        if (G.ord == 2) {
-          if constexpr (KIND == 0) { gx = fx4[2]; gy = fy4[2]; }
-          else { gx = dx4(qk); gy = dy4(qk); }
-          gz = C.d12[2] * (Z(-2) - A(8) * Z(-1) + A(8) * Z(1) - Z(2));
-        } else if (G.ord == 1) {
-          if constexpr (KIND == 0) { gx = fx2[1]; gy = fy2[1]; }
-          else { gx = dx2(qk); gy = dy2(qk); }
-          gz = C.d2[2] * (-Z(-1) + Z(1));
-        }
-        dstore(d + og + 0 * kDTile, (T)gx);
-        dstore(d + og + 1 * kDTile, (T)gy);
-        dstore(d + og + 2 * kDTile, (T)gz);
-      }
-      if constexpr (KIND == 0) {
-        A hxx = A(0), hxy = A(0), hxz = A(0), hyy = A(0), hyz = A(0), hzz = A(0);
-        const A F16 = A(16), F30 = A(30), F8 = A(8), TWO = A(2);
-        if (G.ord == 2) {
-          hxx = C.Fdd[0] * (-X(-2) + F16 * X(-1) - F30 * X(0) - X(2) + F16 * X(1));
-          hyy = C.Fdd[1] * (-Y(-2) + F16 * Y(-1) - F30 * Y(0) - Y(2) + F16 * Y(1));
-          hzz = C.Fdd[2] * (-Z(-2) + F16 * Z(-1) - F30 * Z(0) - Z(2) + F16 * Z(1));
-          auto row = [&](int ob) {
-            const A* r = qk + ob * DSX;
-            return r[-2] - F8 * r[-1] + F8 * r[1] - r[2];
-          };
-          hxy = C.Fxy * (row(-2) - F8 * row(-1) + F8 * row(1) - row(2));
-          hxz = C.d12[2] * (fx4[0] - F8 * fx4[1] + F8 * fx4[3] - fx4[4]);
-          hyz = C.d12[2] * (fy4[0] - F8 * fy4[1] + F8 * fy4[3] - fy4[4]);
-        } else if (G.ord == 1) {
-          hxx = C.Sdd[0] * (X(-1) - TWO * X(0) + X(1));
-          hyy = C.Sdd[1] * (Y(-1) - TWO * Y(0) + Y(1));
-          hzz = C.Sdd[2] * (Z(-1) - TWO * Z(0) + Z(1));
-          hxy = C.Sxy * (qk[-1 - DSX] - qk[1 - DSX] - qk[-1 + DSX] + qk[1 + DSX]);
-          hxz = C.d2[2] * (-fx2[0] + fx2[2]);
-          hyz = C.d2[2] * (-fy2[0] + fy2[2]);
-        }
-        dstore(d + oh + 0 * kDTile, (T)hxx);
-        dstore(d + oh + 1 * kDTile, (T)hxy);
-        dstore(d + oh + 2 * kDTile, (T)hxz);
-        dstore(d + oh + 3 * kDTile, (T)hyy);
-        dstore(d + oh + 4 * kDTile, (T)hyz);
-        dstore(d + oh + 5 * kDTile, (T)hzz);
-      }
-      A adv = A(0);
-      if (G.lop) {
-        // the shift at the point, from the stage input (bsh: its FP64 side
-        // slots in the mixed form), rounded to the storage type T of the
-        // other fields as the pointwise pass sees it
-        const T bx = bsh ? (T)__ldg(bsh + p) : (T)__ldg(in + F_BETAX * fs + p);
-        const T by = bsh ? (T)__ldg(bsh + fs + p) : (T)__ldg(in + F_BETAY * fs + p);
-        const T bz = bsh ? (T)__ldg(bsh + 2 * fs + p) : (T)__ldg(in + F_BETAZ * fs + p);
-        auto Xp = [&](int dd) { return X(dd) + add1; };
-        auto Yp = [&](int dd) { return Y(dd) + add1; };
-        auto Zp = [&](int dd) { return Z(dd) + add1; };
-        adv = lop_term<A>(Xp, (A)bx, (A)bx * C.d12[0], i, G.lo3[0], G.hi[0]);
-        adv = adv + lop_term<A>(Yp, (A)by, (A)by * C.d12[1], j, G.lo3[1], G.hi[1]);
-        adv = adv + lop_term<A>(Zp, (A)bz, (A)bz * C.d12[2], k, G.lo3[2], G.hi[2]);
-      }
-      if (G.ko) {
-        // Z4c dissipates the full diagonal metric d + 1 (Z4c_rhs.f90:1240-1245)
-        const bool ko1 = B.nf == NFIELDS_Z4C && (F == F_GXX || F == F_GYY || F == F_GZZ);
-        A ks;
-        if (ko1)
-          ks = kodiv(ko_sum_rn<A, true>(X), C, 0) + kodiv(ko_sum_rn<A, true>(Y), C, 1) +
-               kodiv(ko_sum_rn<A, true>(Z), C, 2);
-        else
-          ks = kodiv(ko_sum_rn<A, false>(X), C, 0) + kodiv(ko_sum_rn<A, false>(Y), C, 1) +
-               kodiv(ko_sum_rn<A, false>(Z), C, 2);
-        adv = adv + C.ko * ks;
-      }
-      dstore(d + oa, (T)adv);
-    }
-    // slide the register windows
-#pragma unroll
-    for (int t = 0; t < 6; ++t) c[t] = c[t + 1];
-    if constexpr (KIND == 0) {
-#pragma unroll
-      for (int t = 0; t < 4; ++t) { fx4[t] = fx4[t + 1]; fy4[t] = fy4[t + 1]; }
-#pragma unroll
-      for (int t = 0; t < 2; ++t) { fx2[t] = fx2[t + 1]; fy2[t] = fy2[t + 1]; }
-    }
-    // plane k+4 is complete for the next iteration: it replaced plane k-1
-    // (register form) or landed (cp.async form), and no thread reads that slot
-    // in this iteration
-    if constexpr (kAsync) {
-      cp_async_wait<1>();
-      PA.fix(k + 4, ring + rs(k + 4) * DPLANE);
-    } else {
-      P.store(ring + ring_slot(k + 4) * DPLANE, np);
-    }
-    __syncthreads();
+    cp_async_wait<0>();
+    P.land(kA + 3, first(3), land + DPER * DTHREADS);
+    P.issue(kA + 4, nullptr, land);
+    cp_async_commit();
   }
-  // the copies still in flight land before the ring is reused
-  if constexpr (kAsync) cp_async_wait<0>();
+  __syncthreads();
+
+  const A F8 = A(8);
+  const int kE = KIND == 0 ? k1 + 2 : k1;
+  const int cx = lop_codes(i, lox, ex0 - 1), cy0 = lop_codes(j, loy, ex1 - 1), cy1 = lop_codes(j + 1, loy, ex1 - 1);
+  // element offsets of the slots of planes k-3 .. k+5 (k-3, k-2 of the first plane: any)
+  int so[DRING];
+#pragma unroll
+  for (int m = 0; m < DRING; ++m) so[m] = ((m + DRING - 3) % DRING) * DPLANE;
+#pragma unroll 1
+  for (int k = kA; k < kE; ++k) {
+    const int par = (k - kA + 5) & 1;            // landing buffer of k+5
+    P.issue(k + 5, ring + so[8], land + par * (DPER * DTHREADS));
+    shift(k + 2);
+    cp_async_commit();
+    const A* q = ring + so[3] + own;
+    const bool outp = k >= k0 && k < k1 && !((fm & 4) && k == ex2 - 1) && !((fm & 32) && k == 0);
+    if (any && outp) {
+      const int fz = fits_z(k), cz = lop_codes(k, loz, ex2 - 1);
+      const int f0 = fit0 & fz, f1 = fit1 & fz;
+      T* d0 = dptr(0, k);
+      T* d1 = dptr(1, k);
+      A X0[7], X1[7], Y[8];   // x-lines of the two points; the y-line from row -3 to row 4
+#pragma unroll
+      for (int o = -3; o <= 3; ++o)
+        { X0[3 + o] = q[o]; X1[3 + o] = q[DS + o]; }
+#pragma unroll
+      for (int r = -3; r <= 4; ++r) Y[3 + r] = r == 0 ? X0[3] : r == 1 ? X1[3] : q[r * DS];
+      A c0[7], c1[7];         // z-lines
+#pragma unroll
+      for (int m = 0; m < 7; ++m) {
+        c0[m] = m == 3 ? X0[3] : ring[so[m] + own];
+        c1[m] = m == 3 ? X1[3] : ring[so[m] + own + DS];
+      }
+      // 4th-order stencils; points where they do not fit are stored over below
+      if constexpr (KIND == 0) {
+        // row differences f(-2) - 8 f(-1) + 8 f(1) - f(2) of rows -2 .. 3
+        A ds[6];
+        auto row = [&](int r) {
+          const A* u = q + r * DS;
+          return u[-2] - F8 * u[-1] + F8 * u[1] - u[2];
+        };
+        ds[0] = row(-2); ds[1] = row(-1); ds[4] = row(2); ds[5] = row(3);
+        ds[2] = X0[1] - F8 * X0[2] + F8 * X0[4] - X0[5];
+        ds[3] = X1[1] - F8 * X1[2] + F8 * X1[4] - X1[5];
+        wx0[4] = C.d12[0] * ds[2];
+        wx1[4] = C.d12[0] * ds[3];
+        wy0[4] = C.d12[1] * (Y[1] - F8 * Y[2] + F8 * Y[4] - Y[5]);
+        wy1[4] = C.d12[1] * (Y[2] - F8 * Y[3] + F8 * Y[5] - Y[6]);
+        auto dd = [&](A fm2, A fm1, A f0, A f1, A f2, A cf) {
+          return cf * (-fm2 + A(16) * fm1 - A(30) * f0 - f2 + A(16) * f1);
+        };
+        if (m0) {
+          dstore(d0 + og, (T)wx0[4]);
+          dstore(d0 + og + kDTile, (T)wy0[4]);
+          dstore(d0 + oh, (T)dd(X0[1], X0[2], X0[3], X0[4], X0[5], C.Fdd[0]));
+          dstore(d0 + oh + 1 * kDTile, (T)(C.Fxy * (ds[0] - F8 * ds[1] + F8 * ds[3] - ds[4])));
+          dstore(d0 + oh + 3 * kDTile, (T)dd(Y[1], Y[2], Y[3], Y[4], Y[5], C.Fdd[1]));
+          dstore(d0 + oh + 5 * kDTile, (T)dd(c0[1], c0[2], c0[3], c0[4], c0[5], C.Fdd[2]));
+        }
+        if (m1) {
+          dstore(d1 + og, (T)wx1[4]);
+          dstore(d1 + og + kDTile, (T)wy1[4]);
+          dstore(d1 + oh, (T)dd(X1[1], X1[2], X1[3], X1[4], X1[5], C.Fdd[0]));
+          dstore(d1 + oh + 1 * kDTile, (T)(C.Fxy * (ds[1] - F8 * ds[2] + F8 * ds[4] - ds[5])));
+          dstore(d1 + oh + 3 * kDTile, (T)dd(Y[2], Y[3], Y[4], Y[5], Y[6], C.Fdd[1]));
+          dstore(d1 + oh + 5 * kDTile, (T)dd(c1[1], c1[2], c1[3], c1[4], c1[5], C.Fdd[2]));
+        }
+      }
+      if constexpr (KIND == 1) {
+        if (m0) {
+          dstore(d0 + og, (T)(C.d12[0] * (X0[1] - F8 * X0[2] + F8 * X0[4] - X0[5])));
+          dstore(d0 + og + kDTile, (T)(C.d12[1] * (Y[1] - F8 * Y[2] + F8 * Y[4] - Y[5])));
+        }
+        if (m1) {
+          dstore(d1 + og, (T)(C.d12[0] * (X1[1] - F8 * X1[2] + F8 * X1[4] - X1[5])));
+          dstore(d1 + og + kDTile, (T)(C.d12[1] * (Y[2] - F8 * Y[3] + F8 * Y[5] - Y[6])));
+        }
+      }
+      if constexpr (KIND <= 1) {
+        if (m0) dstore(d0 + og + 2 * kDTile, (T)(C.d12[2] * (c0[1] - F8 * c0[2] + F8 * c0[4] - c0[5])));
+        if (m1) dstore(d1 + og + 2 * kDTile, (T)(C.d12[2] * (c1[1] - F8 * c1[2] + F8 * c1[4] - c1[5])));
+      }
+      auto adv = [&](const auto& fX, const auto& fY, const auto& fZ, int a, int cy, int fit) -> A {
+        const double* sb = bet + ((k % DBETA) * 6 + a) * DTHREADS;
+        auto line = [&](const auto& f, int d, int codes) {
+          const A bv = (A)(T)sb[2 * d * DTHREADS];   // rounded as the pointwise pass sees it
+          const A bd = bv * C.d12[d];
+          if constexpr (KIND == 0 && sizeof(A) == 8) return lop_term<A>([&](int o) { return f(o) + add1; }, bv, bd, codes);
+          else return lop_term<A>(f, bv, bd, codes);
+        };
+        const A r = line(fX, 0, cx) + line(fY, 1, cy) + line(fZ, 2, cz);
+        const A ko = C.ko * ko_term<A, Z4C && KIND == 0>(fX, fY, fZ, add1, C);
+        return ((fit & 8) ? r : A(0)) + ((fit & 4) ? ko : A(0));
+      };
+      const A a0 = adv([&](int o) { return X0[3 + o]; }, [&](int o) { return Y[3 + o]; },
+                       [&](int o) { return c0[3 + o]; }, 0, cy0, f0);
+      if (m0) dstore(d0 + oa, (T)a0);
+      const A a1 = adv([&](int o) { return X1[3 + o]; }, [&](int o) { return Y[4 + o]; },
+                       [&](int o) { return c1[3 + o]; }, 1, cy1, f1);
+      if (m1) dstore(d1 + oa, (T)a1);
+      if constexpr (KIND <= 1) {
+        // next to an edge the derivatives are of 2nd order, on it zero.  One
+        // copy of the code for both points
+        if ((m0 && !(f0 & 1)) || (m1 && !(f1 & 1))) {
+#pragma unroll 1
+          for (int a = 0; a < 2; ++a) {
+            const int fit = a ? f1 : f0;
+            if (!(a ? m1 : m0) || (fit & 1)) continue;
+            const A* u = q + a * DS;
+            const A* um = ring + so[2] + own + a * DS;   // planes k-1, k+1
+            const A* up = ring + so[4] + own + a * DS;
+            T* d = a ? d1 : d0;
+            auto put = [&](int o, A v) { dstore(d + o, (fit & 2) ? (T)v : T(0)); };
+            put(og, C.d2[0] * (-u[-1] + u[1]));
+            put(og + kDTile, C.d2[1] * (-u[-DS] + u[DS]));
+            put(og + 2 * kDTile, C.d2[2] * (-um[0] + up[0]));
+            if constexpr (KIND == 0) {
+              const A TWO = A(2), f = u[0];
+              put(oh, C.Sdd[0] * (u[-1] - TWO * f + u[1]));
+              put(oh + 1 * kDTile, C.Sxy * (u[-1 - DS] - u[1 - DS] - u[-1 + DS] + u[1 + DS]));
+              put(oh + 2 * kDTile, C.d2[2] * (-(C.d2[0] * (-um[-1] + um[1])) + C.d2[0] * (-up[-1] + up[1])));
+              put(oh + 3 * kDTile, C.Sdd[1] * (u[-DS] - TWO * f + u[DS]));
+              put(oh + 4 * kDTile, C.d2[2] * (-(C.d2[1] * (-um[-DS] + um[DS])) + C.d2[1] * (-up[-DS] + up[DS])));
+              put(oh + 5 * kDTile, C.Sdd[2] * (um[0] - TWO * f + up[0]));
+            }
+          }
+        }
+      }
+    } else if constexpr (KIND == 0) {
+      if (any) {   // a plane of the windows only
+        auto dx4 = [&](const A* u) { return C.d12[0] * (u[-2] - F8 * u[-1] + F8 * u[1] - u[2]); };
+        auto dy4 = [&](const A* u) { return C.d12[1] * (u[-2 * DS] - F8 * u[-DS] + F8 * u[DS] - u[2 * DS]); };
+        wx0[4] = dx4(q); wy0[4] = dy4(q);
+        wx1[4] = dx4(q + DS); wy1[4] = dy4(q + DS);
+      }
+    }
+    if constexpr (KIND == 0) {
+      // the mixed xz, yz derivatives of plane k-2 where they are of 4th order
+      const int kl = k - 2;
+      if (kl >= k0 && !((fm & 4) && kl == ex2 - 1) && !((fm & 32) && kl == 0)) {
+        const int fz = fits_z(kl);
+        if (m0 && (fit0 & fz & 1)) {
+          T* d = dptr(0, kl) + oh;
+          dstore(d + 2 * kDTile, (T)(C.d12[2] * (wx0[0] - F8 * wx0[1] + F8 * wx0[3] - wx0[4])));
+          dstore(d + 4 * kDTile, (T)(C.d12[2] * (wy0[0] - F8 * wy0[1] + F8 * wy0[3] - wy0[4])));
+        }
+        if (m1 && (fit1 & fz & 1)) {
+          T* d = dptr(1, kl) + oh;
+          dstore(d + 2 * kDTile, (T)(C.d12[2] * (wx1[0] - F8 * wx1[1] + F8 * wx1[3] - wx1[4])));
+          dstore(d + 4 * kDTile, (T)(C.d12[2] * (wy1[0] - F8 * wy1[1] + F8 * wy1[3] - wy1[4])));
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        wx0[t] = wx0[t + 1]; wy0[t] = wy0[t + 1];
+        wx1[t] = wx1[t + 1]; wy1[t] = wy1[t + 1];
+      }
+    }
+    // plane k+4 lands in a slot no thread reads in this step
+    cp_async_wait<1>();
+    P.land(k + 4, ring + so[7], land + (par ^ 1) * (DPER * DTHREADS));
+    __syncthreads();
+    const int s0 = so[0];
+#pragma unroll
+    for (int m = 0; m < DRING - 1; ++m) so[m] = so[m + 1];
+    so[DRING - 1] = s0;
+  }
+  cp_async_wait<0>();   // the copies still in flight land before the ring is reused
 }
 
-// Stencil pass over a work list of (block, tile, field) items, ordered by
-// field so that resident CTAs share one code path.
-template <typename T, typename SI, int MINB>
-__global__ void __launch_bounds__(DTHREADS, MINB) k_deriv(const StepBlock<T>* __restrict__ blocks,
-                                                      const DerivItem* __restrict__ items, int nitems, int sub,
-                                                      T* __restrict__ D, int slots, int region) {
+// Stencil pass over a work list of (block, tile, slab, field) items, ordered
+// by field so that resident CTAs share one code path.
+#ifndef AMSS_DMINB
+#define AMSS_DMINB 2
+#endif
+template <typename T, typename SI, bool Z4C>
+__global__ void __launch_bounds__(DTHREADS, AMSS_DMINB) k_deriv(const StepBlock<T>* __restrict__ blocks,
+                                                       const DerivItem* __restrict__ items, int nitems, int sub,
+                                                       T* __restrict__ D, int slots, int region) {
   extern __shared__ __align__(16) unsigned char smem[];
-  // the two-CTA form fills its ring by cp.async; the forms with more CTAs keep
-  // the register path, whose smaller ring leaves L1 to their spills
-  constexpr bool kAsyncForm = AMSS_DERIV_ASYNC && MINB == kDerivMinbLow;
   for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
     const DerivItem it = items[w];
     const StepBlock<T>& B = blocks[it.block];
@@ -534,44 +575,35 @@ __global__ void __launch_bounds__(DTHREADS, MINB) k_deriv(const StepBlock<T>* __
         // wide fields of the mixed form: FP64 source (state, or the FP64 side stage) and arithmetic
         const double* src = sizeof(SI) == 4 ? B.side[sub == 2 ? 1 : 0] + side_slot(F) * fs
                                             : (const double*)in + F * fs;
-        deriv_column<double, 0, kAsyncForm>(B, src, in, bsh, F, it, D, slots, region, reinterpret_cast<double*>(smem));
+        deriv_march<double, 0, Z4C>(B, src, in, bsh, F, it, D, slots, region, smem);
         __syncthreads();
         continue;
       }
     }
     const SI* src = in + F * fs;
     switch (dkind(F)) {
-      case 0: deriv_column<T, 0, kAsyncForm>(B, src, in, bsh, F, it, D, slots, region, reinterpret_cast<T*>(smem)); break;
-      case 1: deriv_column<T, 1, kAsyncForm>(B, src, in, bsh, F, it, D, slots, region, reinterpret_cast<T*>(smem)); break;
-      default: deriv_column<T, 2, kAsyncForm>(B, src, in, bsh, F, it, D, slots, region, reinterpret_cast<T*>(smem)); break;
+      case 0: deriv_march<T, 0, Z4C>(B, src, in, bsh, F, it, D, slots, region, smem); break;
+      case 1: deriv_march<T, 1, Z4C>(B, src, in, bsh, F, it, D, slots, region, smem); break;
+      default: deriv_march<T, 2, Z4C>(B, src, in, bsh, F, it, D, slots, region, smem); break;
     }
     __syncthreads();
   }
 }
 
-// Shared memory of k_deriv: the plane ring in the widest arithmetic type, for
-// the two-CTA form (cp.async ring) and the others (register path).
-constexpr size_t kDerivSmemLow = (size_t)(AMSS_DERIV_ASYNC ? DRING_ASYNC : DRING) * DPLANE * sizeof(double);
-constexpr size_t kDerivSmem = (size_t)DRING * DPLANE * sizeof(double);
-
 // Stencil pass launcher: substep 0 reads the FP64 state, 1-3 the stages;
-// region: the D order of the points (-1: whole arrays, else StepBlock::rlo);
-// occ selects the compiled occupancy (0: two resident CTAs, 1: more).
+// region: the D order of the points (-1: whole arrays, else StepBlock::rlo).
 template <typename T, typename SS>
 cudaError_t launch_deriv(const void* blocks, const DerivItem* items, int nitems, int sub, void* D, int slots,
-                         int region, int grid, cudaStream_t s, int occ) {
+                         int region, int grid, cudaStream_t s) {
   const StepBlock<T>* bl = (const StepBlock<T>*)blocks;
-  // both < 48 KB: no opt-in attribute needed
-  const size_t smem = occ ? kDerivSmem : kDerivSmemLow;
-  constexpr int hi = sizeof(T) == 8 ? AMSS_DERIV_MINB_F64 : AMSS_DERIV_MINB_F32;
-  if (sub == 0) {
-    if (occ) k_deriv<T, double, hi><<<grid, DTHREADS, smem, s>>>(bl, items, nitems, sub, (T*)D, slots, region);
-    else k_deriv<T, double, kDerivMinbLow><<<grid, DTHREADS, smem, s>>>(bl, items, nitems, sub, (T*)D, slots, region);
-  } else {
-    if (occ) k_deriv<T, SS, hi><<<grid, DTHREADS, smem, s>>>(bl, items, nitems, sub, (T*)D, slots, region);
-    else k_deriv<T, SS, kDerivMinbLow><<<grid, DTHREADS, smem, s>>>(bl, items, nitems, sub, (T*)D, slots, region);
-  }
-  return cudaGetLastError();
+  auto go = [&](auto kernel) -> cudaError_t {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDerivSmem);
+    if (e != cudaSuccess) return e;
+    kernel<<<grid, DTHREADS, kDerivSmem, s>>>(bl, items, nitems, sub, (T*)D, slots, region);
+    return cudaGetLastError();
+  };
+  if (slots == D_SLOTS_Z4C) return sub == 0 ? go(k_deriv<T, double, true>) : go(k_deriv<T, SS, true>);
+  return sub == 0 ? go(k_deriv<T, double, false>) : go(k_deriv<T, SS, false>);
 }
 
 }  // namespace amss

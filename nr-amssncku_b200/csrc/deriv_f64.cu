@@ -2,6 +2,5 @@
 #include "deriv.cuh"
 
 namespace amss {
-template cudaError_t launch_deriv<double, double>(const void*, const DerivItem*, int, int, void*, int, int, int, cudaStream_t,
-                                          int);
+template cudaError_t launch_deriv<double, double>(const void*, const DerivItem*, int, int, void*, int, int, int, cudaStream_t);
 }  // namespace amss

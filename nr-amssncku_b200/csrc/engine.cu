@@ -41,7 +41,7 @@ cudaError_t launch_face(const void* blocks, const int2* faces, int nfaces, int s
                         unsigned* status, cudaStream_t s);
 template <typename T, typename SS>
 cudaError_t launch_deriv(const void* blocks, const DerivItem* items, int nitems, int sub, void* D, int slots,
-                         int region, int grid, cudaStream_t s, int occ);
+                         int region, int grid, cudaStream_t s);
 cudaError_t launch_enforce(long long n, long long fs, double* g, double* a, cudaStream_t s);
 template <typename T>
 cudaError_t launch_constraints(const void* table, const int2* tiles, int ntiles, int tile_pts, bool symm,
@@ -261,18 +261,6 @@ extern "C" int amss_engine_add_amr_block(amss_engine* e, int level, int patch, c
   return (int)e->blocks.size() - 1;
 }
 
-// Stencil-pass tile width of a block of x extent ex0 on level L: the level's
-// tuned width where one is set (at most the block's extent), else deriv_tile_w.
-static int level_tile_w(const ELevel& L, int ex0) {
-  return L.tile_w > 0 ? std::min(L.tile_w, ex0) : deriv_tile_w(ex0);
-}
-
-// Stencil-pass work items of a level: one per (field, x-y tile, z-slab),
-// field-major and grouped by stencil kind (the FP64 fields of the mixed form
-// first), so resident CTAs of the stencil pass run the same code.  A block's
-// z extent is cut into L.zsplit slabs of near-equal height (each slab marches
-// its own planes after a 7-plane prologue): more, shorter work items for
-// levels whose items would otherwise fill the last wave of CTAs poorly.
 // The cells of a block a list covers: 0 its array, 1 its owned cells, 2 its
 // final-substep region (global level indices).
 static Box list_box(const amss_engine* e, const ELevel& L, const EBlock& b, int mode) {
@@ -283,39 +271,28 @@ static Box list_box(const amss_engine* e, const ELevel& L, const EBlock& b, int 
 
 // Stencil-pass work items over each of this rank's blocks of a level: over its
 // array (mode 0), its owned cells (1) or its final-substep region (2); x-y tiles
-// of the level's tile width, z-slabs, ordered by field.
+// (deriv_tile), z-slabs of near-equal height (each marches its own planes after
+// a 4-plane warm-up), ordered by field, so that resident CTAs run the same
+// code, the fields with most stencils first.
 static std::vector<DerivItem> deriv_items(amss_engine* e, const ELevel& L, int mode = 0) {
   static const int order[25] = {F_CHI, F_LAP, F_BETAX, F_BETAY, F_BETAZ, F_GXX, F_GXY, F_GXZ,
                                 F_GYY, F_GYZ, F_GZZ, F_TRK, F_GAMX, F_GAMY, F_GAMZ, F_TZ, F_AXX,
                                 F_AXY, F_AXZ, F_AYY, F_AYZ, F_AZZ, F_DTSFX, F_DTSFY, F_DTSFZ};
   std::vector<DerivItem> tiles;
-  for (size_t m = 0; m < L.own.size(); ++m) {
-    const EBlock& b = e->blocks[L.own[m]];
-    if (mode == 0) {
-      const int tw = level_tile_w(L, b.ex[0]), th = DTHREADS / tw;
-      const int ns = std::max(1, std::min(L.zsplit, b.ex[2] / kMinSlab));
-      for (int z = 0; z < ns; ++z) {
-        const int k0 = ns == 1 ? 0 : (int)((long long)b.ex[2] * z / ns);
-        const int k1 = ns == 1 ? 0 : (int)((long long)b.ex[2] * (z + 1) / ns);
-        for (int y0 = 0; y0 < b.ex[1]; y0 += th)
-          for (int x0 = 0; x0 < b.ex[0]; x0 += tw) tiles.push_back(DerivItem{(int)m, x0, y0, 0, k0, k1});
-      }
-      continue;
+  auto cut = [&](int slabs, int least) {
+    tiles.clear();
+    for (size_t m = 0; m < L.own.size(); ++m) {
+      const EBlock& b = e->blocks[L.own[m]];
+      const Box r = list_box(e, L, b, mode);
+      if (r.empty()) continue;
+      int lo[3], n[3];
+      for (int d = 0; d < 3; ++d) { lo[d] = r.lo[d] - b.org[d]; n[d] = r.hi[d] - r.lo[d]; }
+      deriv_push(tiles, (int)m, lo, n, L.tile_w > 0 ? L.tile_w : DWMAX, slabs, least);
     }
-    const Box r = list_box(e, L, b, mode);
-    if (r.empty()) continue;
-    int lo[3], n[3];
-    for (int d = 0; d < 3; ++d) { lo[d] = r.lo[d] - b.org[d]; n[d] = r.hi[d] - r.lo[d]; }
-    // a region narrower than the smallest tile keeps the block's tile, clipped
-    const int tw = n[0] >= kDerivMinEx ? level_tile_w(L, n[0]) : level_tile_w(L, b.ex[0]), th = DTHREADS / tw;
-    const int ns = std::max(1, std::min(L.zsplit, n[2] / kMinSlab));
-    for (int z = 0; z < ns; ++z) {
-      const int k0 = lo[2] + (int)((long long)n[2] * z / ns), k1 = lo[2] + (int)((long long)n[2] * (z + 1) / ns);
-      for (int y0 = lo[1]; y0 < lo[1] + n[1]; y0 += th)
-        for (int x0 = lo[0]; x0 < lo[0] + n[0]; x0 += tw)
-          tiles.push_back(DerivItem{(int)m, x0, y0, 0, k0, k1, lo[0] + n[0], lo[1] + n[1], tw});
-    }
-  }
+  };
+  cut(L.zsplit, kMinSlab);
+  if (L.tile_w == 0 && L.zsplit == 1)   // untuned
+    cut(deriv_slabs(tiles, e->nf == NFIELDS_Z4C, 2 * e->sm_count), kAutoSlab);
   std::vector<DerivItem> items;
   for (int f : order) {
     if (f == F_TZ && e->nf != NFIELDS_Z4C) continue;
@@ -361,7 +338,6 @@ static int build_table(amss_engine* e, ELevel& L, int level) {
     s.npts = b.npts;
     s.lev0 = level == 0 ? 1 : 0;
     s.nf = e->nf;
-    s.dw = level_tile_w(L, b.ex[0]);
     for (int g = 0; g < 2; ++g) {
       const Box r = list_box(e, L, b, g == 0 ? 2 : 1);
       for (int d = 0; d < 3; ++d) {
@@ -813,8 +789,8 @@ static int step_level_impl(amss_engine* e, int level, double dt, bool fin = fals
     if (split && nditems) {
       const int slots = e->nf == NFIELDS_Z4C ? D_SLOTS_Z4C : D_SLOTS, region = reg ? 0 : own ? 1 : -1;
       const cudaError_t ed =
-          mixed ? launch_deriv<float, float>(L.dtable, ditems, nditems, sub, e->D, slots, region, dgrid, e->stream, L.docc)
-                : launch_deriv<double, double>(L.dtable, ditems, nditems, sub, e->D, slots, region, dgrid, e->stream, L.docc);
+          mixed ? launch_deriv<float, float>(L.dtable, ditems, nditems, sub, e->D, slots, region, dgrid, e->stream)
+                : launch_deriv<double, double>(L.dtable, ditems, nditems, sub, e->D, slots, region, dgrid, e->stream);
       AMSS_CK(ed);
       e->launches++;
     }
@@ -899,21 +875,11 @@ static int recursive_step(amss_engine* e, int l, double dt0) {
   return 0;
 }
 
-template <typename T>
-static int patch_table_dw(amss_engine* e, ELevel& L) {
-  for (size_t m = 0; m < L.own.size(); ++m) {
-    const int dw = level_tile_w(L, e->blocks[L.own[m]].ex[0]);
-    char* dst = (char*)L.dtable + m * sizeof(StepBlock<T>) + offsetof(StepBlock<T>, dw);
-    AMSS_CK(cudaMemcpy(dst, &dw, sizeof(int), cudaMemcpyHostToDevice));
-  }
-  return 0;
-}
-
 extern "C" int amss_engine_set_level_tiling(amss_engine* e, int level, int tile_w, int zsplit) {
   if (!e || !e->committed || e->plan_only) return amss_fail(AMSS_ERR_STATE, "engine not committed");
   auto it = e->levels.find(level);
   if (it == e->levels.end()) return amss_fail(AMSS_ERR_ARG, "amss_engine_set_level_tiling: no such level");
-  if (tile_w != 0 && (tile_w < kDerivMinEx || tile_w > DWMAX))
+  if (tile_w != 0 && (tile_w < kDerivMinEx || tile_w > kMaxTileW))
     return amss_fail(AMSS_ERR_ARG, "amss_engine_set_level_tiling: tile width must be 0 or 8..64");
   if (zsplit < 1 || zsplit > 16) return amss_fail(AMSS_ERR_ARG, "amss_engine_set_level_tiling: zsplit must be 1..16");
   ELevel& L = it->second;
@@ -941,7 +907,7 @@ extern "C" int amss_engine_set_level_tiling(amss_engine* e, int level, int tile_
     AMSS_CK(cudaMalloc(&L.ditems_s, items_s.size() * sizeof(DerivItem)));
     AMSS_CK(cudaMemcpy(L.ditems_s, items_s.data(), items_s.size() * sizeof(DerivItem), cudaMemcpyHostToDevice));
   }
-  return e->prm.precision == 1 ? patch_table_dw<float>(e, L) : patch_table_dw<double>(e, L);
+  return 0;
 }
 
 extern "C" int amss_engine_level_final_region(amss_engine* e, int level, int* pad, long long* points) {

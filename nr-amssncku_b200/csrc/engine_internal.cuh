@@ -137,7 +137,7 @@ struct ELevel {
   int ntiles_s = 0;
   DerivItem* ditems_s = nullptr;   // and the stencil-pass items
   int nditems_s = 0;
-  int tile_w = 0;               // stencil-pass tile width (0: deriv_tile_w of each block's x extent)
+  int tile_w = 0;               // stencil-pass tile width as set (0: default; at most DWMAX is used)
   int zsplit = 1;               // z-slabs per block in the stencil pass
   int docc = 0;                 // stencil-pass occupancy form: 0 two resident CTAs, 1 more (deriv.cuh)
   int dtiles_n = 0;             // D tiles of this level

@@ -24,8 +24,7 @@ struct Coef {
   T Fxy, Fxz, Fyz;   // (1/144)/(dx*dy)
   T Sxy, Sxz, Syz;   // 0.25/(dx*dy)
   T h[3];            // dx itself (KO divides by it)
-  T hinv[3];         // 1/dx, used instead of the division when every dx is a power of two (exact)
-  int hpow2;
+  T hinv[3];         // 1/dx, rounded
   T ko;              // eps/64
 };
 
@@ -389,11 +388,20 @@ __device__ __forceinline__ T ko_sum_rn(const FN& f) {
   }
 }
 
+// a / dx, as the reference divides.  FP64: the product with the rounded
+// reciprocal, corrected by its remainder (Markstein 1990, "Computation of
+// elementary functions on the IBM RISC System/6000 processor"): the rounded
+// quotient in four operations instead of a division; an infinite quotient,
+// whose remainder is no number, stays as it is.
 template <typename T>
 __device__ __forceinline__ T kodiv(T a, const Coef<T>& c, int d) {
-  // the reference divides by dx; for dx = 2^k the product with 2^-k is the same number
-  if constexpr (sizeof(T) == 8) return c.hpow2 ? a * c.hinv[d] : a / c.h[d];
-  else return a * (T(1) / c.h[d]);
+  if constexpr (sizeof(T) == 8) {
+    const T q = a * c.hinv[d];
+    const T r = fma(fma(-q, c.h[d], a), c.hinv[d], q);
+    return fabs(q) < T(1.7976931348623157e308) ? r : q;
+  } else {
+    return a * c.hinv[d];
+  }
 }
 
 }  // namespace amss
