@@ -24,14 +24,17 @@ struct EpiNone {   // the right-hand side itself is not wanted
 constexpr int kConsThreads = 128;
 
 // residuals of every point of the level into cons (7 fields, the D layout:
-// block offset doff, field stride dfs)
+// block offset doff, field stride dfs).  A CTA a tile: the pass waits on the
+// loads of its stencils at eight warps an SM (255 registers), and a grid of
+// eight CTAs an SM that loops over the tiles leaves a slot empty while a CTA's
+// last warp finishes: 1,037 us for the norms of 102^3 points, 799 us now.
+// (168 registers and three CTAs: 883 us, four: 858 us, for their spills.)
 template <typename T, bool SYMM>
 __global__ void __launch_bounds__(kConsThreads) k_constraints(const StepBlock<T>* __restrict__ blocks,
-                                                              const int2* __restrict__ tiles, int ntiles, int tile_pts,
+                                                              const int2* __restrict__ tiles, int tile_pts,
                                                               double* __restrict__ cons, long long dfs) {
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x)
   for (int e = threadIdx.x; e < tile_pts; e += blockDim.x) {
-    const int2 tile = tiles[t];
+    const int2 tile = tiles[blockIdx.x];
     const StepBlock<T>& B = blocks[tile.x];
     const long long p = (long long)tile.y + e;
     if (p >= B.npts) continue;
@@ -98,11 +101,10 @@ cudaError_t launch_constraints(const void* table, const int2* tiles, int ntiles,
                                const int* region, double* cons, long long dfs, double* part, int grid,
                                cudaStream_t s) {
   const StepBlock<T>* bl = (const StepBlock<T>*)table;
-  const int g1 = ntiles < 148 * 8 ? ntiles : 148 * 8;
   if (symm)
-    k_constraints<T, true><<<g1, kConsThreads, 0, s>>>(bl, tiles, ntiles, tile_pts, cons, dfs);
+    k_constraints<T, true><<<ntiles, kConsThreads, 0, s>>>(bl, tiles, tile_pts, cons, dfs);
   else
-    k_constraints<T, false><<<g1, kConsThreads, 0, s>>>(bl, tiles, ntiles, tile_pts, cons, dfs);
+    k_constraints<T, false><<<ntiles, kConsThreads, 0, s>>>(bl, tiles, tile_pts, cons, dfs);
   k_constraint_sums<T><<<grid, kConsThreads, 0, s>>>(bl, tiles, ntiles, tile_pts, region, cons, dfs, part);
   return cudaGetLastError();
 }

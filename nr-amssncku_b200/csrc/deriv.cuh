@@ -22,8 +22,8 @@
 // from shared memory; stencils that do not fit are chosen by selects or, for
 // the 2nd-order ones next to an edge, stored over the 4th-order ones.  One
 // column a thread with a register column and per-stencil branches, 35 x 7
-// tiles and whole-block marches took 359 us (mixed 293 us, 200 us now; a 24^3
-// block 72 us, 20 us now, cut into z-slabs).  A second, fully gated path beside
+// tiles and whole-block marches took 359 us (mixed 293 us, 226 us now; a 24^3
+// block 74 us, 26 us now, cut into z-slabs).  A second, fully gated path beside
 // a full-width one, in the same warps, was slower (no room in the instruction
 // cache, warps waiting for each other at the plane's barrier).
 //
