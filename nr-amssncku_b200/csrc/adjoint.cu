@@ -192,7 +192,7 @@ int rhs_vjp(amss_adjoint* a, int sub, const double* Xin, const double* Rbv, doub
   k_beta_adjoint<<<grid_of(a->npts), 128, 0, s>>>(a->dadj, a->Db);
   AMSS_CK(cudaGetLastError());
   if (a->nfaces) {
-    k_face_vjp<<<grid_of(a->nfaces), 128, 0, s>>>(a->dadj, a->dfaces, a->nfaces);
+    k_face_vjp<<<dim3(grid_of(a->nfaces), NFIELDS_BSSN), 128, 0, s>>>(a->dadj, a->dfaces, a->nfaces);
     AMSS_CK(cudaGetLastError());
     a->launches++;
   }
