@@ -289,14 +289,23 @@ extern "C" amss_adjoint* amss_adjoint_create(const int ex[3], const double bbox[
   const int slabs = deriv_slabs(cut, false, 2 * 148);
   cut.clear();
   deriv_push(cut, 0, lo, ex, DWMAX, slabs, kAutoSlab);
+  // the transpose's tiles, and its slabs by the same rule (its warm-up and
+  // run-out are six planes too)
+  std::vector<DerivItem> gcut;
+  const int tw = tg_tile_w(ex[0]), th = DTHREADS / tw;
+  for (int y0 = 0; y0 < ex[1]; y0 += th)
+    for (int x0 = 0; x0 < ex[0]; x0 += tw) gcut.push_back(DerivItem{0, x0, y0, 0, 0, ex[2], ex[0], ex[1], tw, th});
+  const int gslabs = std::min(deriv_slabs(gcut, false, 2 * 148), ex[2] / kAutoSlab);
   for (int f : order) {
     for (DerivItem it : cut) {
       it.field = f;
       items.push_back(it);
     }
-    const int tw = tg_tile_w(ex[0]), th = DTHREADS / tw;
-    for (int y0 = 0; y0 < ex[1]; y0 += th)
-      for (int x0 = 0; x0 < ex[0]; x0 += tw) gitems.push_back(TgItem{x0, y0, f});
+    for (const DerivItem& it : gcut) {
+      const int ns = gslabs < 1 ? 1 : gslabs;
+      for (int z = 0; z < ns; ++z)
+        gitems.push_back(TgItem{it.x0, it.y0, f, (int)((long long)ex[2] * z / ns), (int)((long long)ex[2] * (z + 1) / ns)});
+    }
   }
   for (long long p = 0; p < a->npts; p += kPointwiseTile) tiles.push_back(make_int2(0, (int)p));
   const int fm = s.b.face_mask;

@@ -229,8 +229,11 @@ struct TgMap {
 };
 // Its tile is W x H columns, one thread a column: W = the block's x extent cut
 // into pieces of at most 64, H = DTHREADS / W rows.
+// It gathers the output planes [k0, k1): small blocks are cut into z-slabs, each
+// with three planes of sources on either side (46 x 40 x 42 points: 192 CTAs of
+// 45 steps left most of the chip idle, 320 us; 192 us now).
 struct TgItem {
-  int x0, y0, field;
+  int x0, y0, field, k0, k1;
 };
 constexpr int kTgPlane = 704;                          // cells of one staged plane (>= (W+6)(H+6))
 constexpr int kTgPer = (kTgPlane + DTHREADS - 1) / DTHREADS;   // plane cells a thread stages
@@ -319,11 +322,11 @@ __device__ __forceinline__ void tg_prefetch(const AdjBlock& A, const double* Db,
 }
 
 template <int KIND>
-__device__ __forceinline__ void tg_column(const AdjBlock& A, const double* __restrict__ Db, int F, int x0, int y0,
-                                          double* smem) {
+__device__ __forceinline__ void tg_column(const AdjBlock& A, const double* __restrict__ Db, const TgItem& it,
+                                          const Coef<double>& C, const double* kods, double* smem) {
+  const int F = it.field, x0 = it.x0, y0 = it.y0;
   using M = TgMap<KIND>;
   const BlockView& b = A.b;
-  const Coef<double>& C = A.C.t;
   const int ex0 = b.ex[0], ex1 = b.ex[1], ex2 = b.ex[2];
   const int hix = ex0 - 1, hiy = ex1 - 1, hiz = ex2 - 1;
   const int W = tg_tile_w(ex0), H = DTHREADS / W;
@@ -350,14 +353,16 @@ __device__ __forceinline__ void tg_column(const AdjBlock& A, const double* __res
 
   TgCells cells;
   cells.init(x0, y0, DSX, np, ex0, ex1);
-  tg_stage<KIND>(A, Db, s0, 0, cells, smem);
+  // source planes [mb, me) reach the outputs
+  const int mb = it.k0 - 3 > 0 ? it.k0 - 3 : 0, me = it.k1 + 3 < ex2 ? it.k1 + 3 : ex2;
+  tg_stage<KIND>(A, Db, s0, mb, cells, smem + (mb & 1) * 10 * kTgPlane);
   cp_async_commit();
 #pragma unroll 1
-  for (int m = 0; m < ex2 + 3; ++m) {
-    if (m < ex2) {
-      if (m + 1 < ex2) tg_stage<KIND>(A, Db, s0, m + 1, cells, smem + ((m + 1) & 1) * 10 * kTgPlane);
+  for (int m = mb; m < it.k1 + 3; ++m) {
+    if (m < me) {
+      if (m + 1 < me) tg_stage<KIND>(A, Db, s0, m + 1, cells, smem + ((m + 1) & 1) * 10 * kTgPlane);
       cp_async_commit();
-      if (m + 5 < ex2) tg_prefetch<KIND>(A, Db, s0, m + 5, x0, y0, W, H);
+      if (m + 5 < me) tg_prefetch<KIND>(A, Db, s0, m + 5, x0, y0, W, H);
       double gz = 0.0, hzz = 0.0, bz = 0.0;
       if (mine) {
         if (KIND != 2) gz = __ldg(gzc + m * sz);
@@ -376,7 +381,7 @@ __device__ __forceinline__ void tg_column(const AdjBlock& A, const double* __res
           const unsigned pf = d == 0 ? pfx : pfy, pc = d == 0 ? pcx : pcy;
           const int st = d == 0 ? 1 : DSX;
           const int other = (d == 0 ? fby : fbx) & fbz;
-          const double kod = C.ko / C.h[d], lpd = C.d12[d];
+          const double kod = kods[d], lpd = C.d12[d];
 #pragma unroll
           for (int o = -3; o <= 3; ++o) {
             const int f = other & tg_bits(pf, o);
@@ -469,7 +474,7 @@ __device__ __forceinline__ void tg_column(const AdjBlock& A, const double* __res
         {
           const double ab = P[M::ADV * kTgPlane + own];
           const int code = (fq & 8) && bz != 0.0 ? lop_code(bz > 0.0, m, 0, hiz) : 3;
-          const double kod = (fq & 4) ? C.ko / C.h[2] : 0.0;
+          const double kod = (fq & 4) ? kods[2] : 0.0;
           const double lz = bz * C.d12[2];
 #pragma unroll
           for (int o = -3; o <= 3; ++o) {
@@ -481,7 +486,7 @@ __device__ __forceinline__ void tg_column(const AdjBlock& A, const double* __res
       __syncthreads();   // every thread is done with plane m's buffer before plane m+2 is staged into it
     }
     const int k = m - 3;
-    if (k >= 0 && mine) out[k * sz] += acc[0];
+    if (k >= it.k0 && mine) out[k * sz] += acc[0];
 #pragma unroll
     for (int t = 0; t < 6; ++t) acc[t] = acc[t + 1];
     acc[6] = 0.0;
@@ -496,10 +501,18 @@ __global__ void __launch_bounds__(DTHREADS, 2) k_stencil_gather_tiled(const AdjB
   extern __shared__ __align__(16) unsigned char tg_smem[];
   const TgItem it = items[blockIdx.x];
   double* smem = reinterpret_cast<double*>(tg_smem);
+  // the block's coefficients: in global memory they would be read again, and
+  // the KO quotients divided again, after every plane's stores
+  __shared__ Coef<double> C;
+  __shared__ double kods[3];
+  if (threadIdx.x < sizeof(Coef<double>) / 8)
+    reinterpret_cast<double*>(&C)[threadIdx.x] = reinterpret_cast<const double*>(&A->C.t)[threadIdx.x];
+  if (threadIdx.x < 3) kods[threadIdx.x] = A->C.t.ko / A->C.t.h[threadIdx.x];
+  __syncthreads();
   switch (dkind(it.field)) {
-    case 0: tg_column<0>(*A, Db, it.field, it.x0, it.y0, smem); break;
-    case 1: tg_column<1>(*A, Db, it.field, it.x0, it.y0, smem); break;
-    default: tg_column<2>(*A, Db, it.field, it.x0, it.y0, smem); break;
+    case 0: tg_column<0>(*A, Db, it, C, kods, smem); break;
+    case 1: tg_column<1>(*A, Db, it, C, kods, smem); break;
+    default: tg_column<2>(*A, Db, it, C, kods, smem); break;
   }
 }
 
