@@ -238,8 +238,11 @@ extern "C" int compute_rhs_bssn_(
   double* cs[7] = {ham_Res, movx_Res, movy_Res, movz_Res, Gmx_Res, Gmy_Res, Gmz_Res};
   const size_t bytes = (size_t)n * sizeof(double);
   cudaStream_t s = c.stream;
-  for (int f = 0; f < 24; ++f) AMSS_CK(cudaMemcpyAsync(du + f * fs, st_in[f], bytes, cudaMemcpyHostToDevice, s));
-  for (int f = 0; f < 10; ++f) AMSS_CK(cudaMemcpyAsync(dm + f * fs, mat[f], bytes, cudaMemcpyHostToDevice, s));
+  CopyField io[24 + 18 + 6 + 7];
+  int nio = 0;
+  for (int f = 0; f < 24; ++f) io[nio++] = {du + f * fs, st_in[f]};
+  for (int f = 0; f < 10; ++f) io[nio++] = {dm + f * fs, mat[f]};
+  AMSS_CK(copy_fields(c.pool, io, nio, bytes, true, s));
   AMSS_CK(cudaMemcpyAsync(dX, X, ex[0] * sizeof(double), cudaMemcpyHostToDevice, s));
   AMSS_CK(cudaMemcpyAsync(dY, Y, ex[1] * sizeof(double), cudaMemcpyHostToDevice, s));
   AMSS_CK(cudaMemcpyAsync(dZ, Z, ex[2] * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -266,11 +269,13 @@ extern "C" int compute_rhs_bssn_(
   AMSS_CK(cudaMemcpyAsync(&hs, c.dstatus, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
   AMSS_CK(cudaStreamSynchronize(s));
   if ((hs & ST_NAN) || ((hs & ST_PINF) && (hs & ST_NINF))) return 1;  // bssn_rhs.f90:136, outputs untouched
-  for (int f = 0; f < 24; ++f) AMSS_CK(cudaMemcpyAsync(rh[f], dr + f * fs, bytes, cudaMemcpyDeviceToHost, s));
-  for (int f = 0; f < 18; ++f) AMSS_CK(cudaMemcpyAsync(gm[f], dg + f * fs, bytes, cudaMemcpyDeviceToHost, s));
-  for (int f = 0; f < 6; ++f) AMSS_CK(cudaMemcpyAsync(rc[f], dR + f * fs, bytes, cudaMemcpyDeviceToHost, s));
+  nio = 0;
+  for (int f = 0; f < 24; ++f) io[nio++] = {dr + f * fs, rh[f]};
+  for (int f = 0; f < 18; ++f) io[nio++] = {dg + f * fs, gm[f]};
+  for (int f = 0; f < 6; ++f) io[nio++] = {dR + f * fs, rc[f]};
   if (*co == 0)
-    for (int f = 0; f < 7; ++f) AMSS_CK(cudaMemcpyAsync(cs[f], dc + f * fs, bytes, cudaMemcpyDeviceToHost, s));
+    for (int f = 0; f < 7; ++f) io[nio++] = {dc + f * fs, cs[f]};
+  AMSS_CK(copy_fields(c.pool, io, nio, bytes, false, s));
   AMSS_CK(cudaStreamSynchronize(s));
   return 0;
 }
@@ -324,8 +329,11 @@ extern "C" int compute_rhs_z4c_(
   double* cs[7] = {Hcon, Mxcon, Mycon, Mzcon, Gmxcon, Gmycon, Gmzcon};
   const size_t bytes = (size_t)n * sizeof(double);
   cudaStream_t s = c.stream;
-  for (int f = 0; f < 25; ++f) AMSS_CK(cudaMemcpyAsync(du + f * fs, st_in[f], bytes, cudaMemcpyHostToDevice, s));
-  for (int f = 0; f < 10; ++f) AMSS_CK(cudaMemcpyAsync(dm + f * fs, mat[f], bytes, cudaMemcpyHostToDevice, s));
+  CopyField io[25 + 18 + 6 + 7];
+  int nio = 0;
+  for (int f = 0; f < 25; ++f) io[nio++] = {du + f * fs, st_in[f]};
+  for (int f = 0; f < 10; ++f) io[nio++] = {dm + f * fs, mat[f]};
+  AMSS_CK(copy_fields(c.pool, io, nio, bytes, true, s));
   AMSS_CK(cudaMemcpyAsync(dX, X, ex[0] * sizeof(double), cudaMemcpyHostToDevice, s));
   AMSS_CK(cudaMemcpyAsync(dY, Y, ex[1] * sizeof(double), cudaMemcpyHostToDevice, s));
   AMSS_CK(cudaMemcpyAsync(dZ, Z, ex[2] * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -357,10 +365,12 @@ extern "C" int compute_rhs_z4c_(
   RhsAux aux{dg, dR, dc, dm, fs, 0};
   if (b.lowsym_mask) AMSS_CK(launch_rhs_dropin<true>(grid, s, b, C, du, dscr, aux, c.dstatus));
   else AMSS_CK(launch_rhs_dropin<false>(grid, s, b, C, du, dscr, aux, c.dstatus));
-  for (int f = 0; f < 25; ++f) AMSS_CK(cudaMemcpyAsync(rh[f], dr + f * fs, bytes, cudaMemcpyDeviceToHost, s));
-  for (int f = 0; f < 18; ++f) AMSS_CK(cudaMemcpyAsync(gm[f], dg + f * fs, bytes, cudaMemcpyDeviceToHost, s));
-  for (int f = 0; f < 6; ++f) AMSS_CK(cudaMemcpyAsync(rc[f], dR + f * fs, bytes, cudaMemcpyDeviceToHost, s));
-  for (int f = 0; f < 7; ++f) AMSS_CK(cudaMemcpyAsync(cs[f], dc + f * fs, bytes, cudaMemcpyDeviceToHost, s));
+  nio = 0;
+  for (int f = 0; f < 25; ++f) io[nio++] = {dr + f * fs, rh[f]};
+  for (int f = 0; f < 18; ++f) io[nio++] = {dg + f * fs, gm[f]};
+  for (int f = 0; f < 6; ++f) io[nio++] = {dR + f * fs, rc[f]};
+  for (int f = 0; f < 7; ++f) io[nio++] = {dc + f * fs, cs[f]};
+  AMSS_CK(copy_fields(c.pool, io, nio, bytes, false, s));
   AMSS_CK(cudaStreamSynchronize(s));
   return 0;
 }

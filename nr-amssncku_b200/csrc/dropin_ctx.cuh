@@ -6,12 +6,37 @@
 
 namespace amss {
 
+// Pinned pieces and streams of the threaded copies (dropin_copy.cu), made at
+// the first large copy.
+constexpr int kCopyWorkers = 8;
+constexpr size_t kCopyPiece = (size_t)1 << 20;
+struct CopyPool {
+  char* pinned = nullptr;
+  cudaStream_t stream[kCopyWorkers] = {};
+  cudaEvent_t done[kCopyWorkers][2] = {};
+  int device = 0;
+  bool ready = false, failed = false;
+  ~CopyPool();
+  bool init();
+  void release();
+  char* slot(int w, int s) { return pinned + (size_t)(2 * w + s) * kCopyPiece; }
+};
+struct CopyField {
+  void* dev;
+  void* host;
+};
+// Copies `bytes` of every field host -> device or back.  In stream order with
+// s; the threaded form has also completed on return.
+cudaError_t copy_fields(CopyPool& pool, const CopyField* fields, int nfields, size_t bytes, bool to_device,
+                        cudaStream_t s);
+
 // Per-thread device scratch of the drop-in entries (grow-only, reused).
 struct DropinCtx {
   cudaStream_t stream = nullptr;
   double* dbuf = nullptr;
   size_t cap = 0;      // doubles
   unsigned* dstatus = nullptr;
+  CopyPool pool;
   bool ok = false;
   ~DropinCtx() {
     if (dbuf) cudaFree(dbuf);
