@@ -41,7 +41,7 @@ cudaError_t launch_face(const void* blocks, const int2* faces, int nfaces, int s
                         unsigned* status, cudaStream_t s);
 template <typename T, typename SS>
 cudaError_t launch_deriv(const void* blocks, const DerivItem* items, int nitems, int sub, void* D, int slots,
-                         int region, int grid, cudaStream_t s);
+                         int region, int spare, int grid, cudaStream_t s);
 
 // out = E(in) on the metric / A~ fields; other fields copied.
 __global__ void k_enforce_copy(const double* __restrict__ in, double* __restrict__ out, long long n, long long fs) {
@@ -112,8 +112,9 @@ namespace {
 
 size_t state_bytes(const amss_adjoint* a) { return (size_t)NFIELDS_BSSN * a->fs * sizeof(double); }
 
-// values of one array of stencil terms: whole tiles (stencil.cuh)
-size_t dterms(const amss_adjoint* a) { return (size_t)((a->npts + kDTile - 1) / kDTile) * kDTile * D_SLOTS; }
+// tiles of one array of stencil terms (stencil.cuh), and its values with the stencil pass's spare tile
+int dtiles(const amss_adjoint* a) { return (int)((a->npts + kDTile - 1) / kDTile); }
+size_t dterms(const amss_adjoint* a) { return (size_t)(dtiles(a) + 1) * kDTile * D_SLOTS; }
 
 int grid_of(long long n) {
   const long long b = (n + 127) / 128;
@@ -158,7 +159,7 @@ int fwd_step(amss_adjoint* a, const double* U0raw, double* Unew, double* Z0, dou
   for (int sub = 0; sub < 4; ++sub) {
     const StepBlock<double>* T = a->dtab + sub;
     double* D = Dsub ? Dsub[sub] : a->D;
-    AMSS_CK((launch_deriv<double, double>(T, a->ditems, a->nitems, sub, D, D_SLOTS, -1, std::min(a->nitems, 148 * 16), s)));
+    AMSS_CK((launch_deriv<double, double>(T, a->ditems, a->nitems, sub, D, D_SLOTS, -1, dtiles(a), std::min(a->nitems, 148 * 16), s)));
     AMSS_CK((launch_pointwise<double, double, false>(T, a->dtiles, a->ntiles, sub, rk, 0, a->dstatus, s, D)));
     AMSS_CK((launch_face<double, double>(T, a->dfaces, a->nfaces, sub, rk, 0, a->dstatus, s)));
     a->launches += 3;
@@ -177,7 +178,7 @@ int rhs_vjp(amss_adjoint* a, int sub, const double* Xin, const double* Rbv, doub
   cudaStream_t s = a->stream;
   const StepBlock<double>* T = a->dtab + sub;
   if (!Dpre) {
-    AMSS_CK((launch_deriv<double, double>(T, a->ditems, a->nitems, sub, a->D, D_SLOTS, -1, std::min(a->nitems, 148 * 16), s)));
+    AMSS_CK((launch_deriv<double, double>(T, a->ditems, a->nitems, sub, a->D, D_SLOTS, -1, dtiles(a), std::min(a->nitems, 148 * 16), s)));
     a->launches++;
   }
   a->host_adj.D = Dpre ? Dpre : a->D;
@@ -369,7 +370,7 @@ static int loss_and_grad(amss_adjoint* a, double* loss, bool want_grad) {
   const int gw = 3;
   a->host_tab[0].tl[0] = a->U;   // stencil pass of U (substep-0 input)
   AMSS_CK(cudaMemcpyAsync(a->dtab, a->host_tab, sizeof(StepBlock<double>), cudaMemcpyHostToDevice, s));
-  AMSS_CK((launch_deriv<double, double>(a->dtab, a->ditems, a->nitems, 0, a->D, D_SLOTS, -1, std::min(a->nitems, 148 * 16), s)));
+  AMSS_CK((launch_deriv<double, double>(a->dtab, a->ditems, a->nitems, 0, a->D, D_SLOTS, -1, dtiles(a), std::min(a->nitems, 148 * 16), s)));
   a->host_adj.D = a->D;
   a->host_adj.X = a->U;
   a->host_adj.Rb = nullptr;

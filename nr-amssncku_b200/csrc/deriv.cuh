@@ -14,18 +14,22 @@
 // planes late, so that each is formed once.
 //
 // The pass is bound by instruction issue and latency, not by memory (417 MB in
-// 291 us on 70^3 points; of 10,200 instructions a point 2,100 are FP64), so the
+// 264 us on 70^3 points; of 9,000 instructions a point 2,100 are FP64), so the
 // layout serves those: two columns a thread share the row differences of the
 // cross stencil, the y-line, and a step's barrier, gates and addresses; the
 // row stride is a constant, so that a stencil's reads differ by immediates;
 // the shift comes through shared memory two planes ahead, the coefficients
 // from shared memory; stencils that do not fit are chosen by selects or, for
-// the 2nd-order ones next to an edge, stored over the 4th-order ones.  One
-// column a thread with a register column and per-stencil branches, 35 x 7
-// tiles and whole-block marches took 359 us (mixed 293 us, 226 us now; a 24^3
-// block 74 us, 26 us now, cut into z-slabs).  A second, fully gated path beside
-// a full-width one, in the same warps, was slower (no room in the instruction
-// cache, warps waiting for each other at the plane's barrier).
+// the 2nd-order ones next to an edge, stored over the 4th-order ones; points
+// that are not the thread's to store go to a spare tile, so that the step is
+// straight-line code; what the march needs of the block is in registers, as
+// its waits would have it read again.  One column a thread with a register
+// column and per-stencil branches, 35 x 7 tiles and whole-block marches took
+// 359 us (mixed 293 us, 196 us now), two columns with branches for the points'
+// stores and the block read again 291 us (mixed 226 us).  A second, full-width
+// path beside the gated one took 22 % fewer instructions and was slower where
+// tiles hold many edge points (134^3 Z4c +9 %): its warps wait for the others
+// at the plane's barrier.
 //
 // The planes are copied by cp.async into a ring of nine (k-3 .. k+3 in use, k+4
 // landing, k+5 issued), one barrier a plane.  A source that needs conversion
@@ -137,17 +141,18 @@ inline int deriv_slabs(const std::vector<DerivItem>& one, bool z4c, int ctas) {
 // kind of a field's stencil record: 0 gradient + Hessian + adv, 1 gradient + adv, 2 adv
 __host__ __device__ constexpr int dkind(int F) { return dslots(F) == 10 ? 0 : (dslots(F) == 4 ? 1 : 2); }
 
-// Asynchronous copies global -> shared of one 8- or 4-byte cell (zero-filled
-// when !valid; the source address is then not read).
+// Asynchronous copies global -> shared of one 8- or 4-byte cell; zero-filled
+// when !valid (the source address is then not read).
 __device__ __forceinline__ void cp_async8(void* sdst, const void* gsrc, bool valid) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(gsrc), "r"(valid ? 8 : 0)
                : "memory");
 }
-__device__ __forceinline__ void cp_async4(void* sdst, const void* gsrc, bool valid) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(sa), "l"(gsrc), "r"(valid ? 4 : 0)
-               : "memory");
+__device__ __forceinline__ void cp_async8(unsigned sdst, const void* gsrc) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sdst), "l"(gsrc) : "memory");
+}
+__device__ __forceinline__ void cp_async4(unsigned sdst, const void* gsrc) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sdst), "l"(gsrc) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
@@ -197,21 +202,24 @@ struct PlaneCells {
   }
   // whether cell e of plane kk takes the opposite sign of its source
   __device__ __forceinline__ bool flips(int e, int kk) const { return (((neg >> e) & 1u) != 0) != (kk < 0 && (odd & 4)); }
-  // issues the copies of plane kk (negative: mirrored, past the end: 0): into
-  // the ring slot (no conversion), or into buf, one cell per thread and e
+  // issues the copies of plane kk (negative: mirrored): into the ring slot (no
+  // conversion), or into buf, one cell per thread and e.  Cells past the
+  // block's end are set to 0 at once.
   __device__ __forceinline__ void issue(int kk, A* slot, S* buf) const {
     const int k = kk < 0 ? -kk - 1 : kk;
+    const S* pl = src + k * sz;
     const bool kin = k < ex2;
-    const S* pl = src + (kin ? k * sz : 0);
 #pragma unroll
-    for (int e = 0; e < DPER; ++e)
-      if (off[e] >= -1) {
-        const bool ok = kin && off[e] >= 0;
-        const S* g = ok ? pl + off[e] : src;
-        void* d = sizeof(A) == sizeof(S) ? (void*)(slot + pos[e]) : (void*)(buf + threadIdx.x + e * DTHREADS);
-        if constexpr (sizeof(S) == 8) cp_async8(d, g, ok);
-        else cp_async4(d, g, ok);
+    for (int e = 0; e < DPER; ++e) {
+      S* d = sizeof(A) == sizeof(S) ? reinterpret_cast<S*>(slot) + pos[e] : buf + threadIdx.x + e * DTHREADS;
+      if (kin && off[e] >= 0) {
+        const unsigned sa = (unsigned)__cvta_generic_to_shared(d);
+        if constexpr (sizeof(S) == 8) cp_async8(sa, pl + off[e]);
+        else cp_async4(sa, pl + off[e]);
+      } else if (off[e] >= -1) {
+        *d = S(0);
       }
+    }
   }
   // once this thread's copies of plane kk landed: their signs, and the conversion
   __device__ __forceinline__ void land(int kk, A* slot, const S* buf) const {
@@ -255,18 +263,10 @@ __device__ __forceinline__ A lop_term(const FN& f, A b, A bd, int codes) {
   return r;
 }
 
-// KO dissipation of a point from its three lines, each taken with `add` added
-// (Z4C: 1 for the diagonal metric, Z4c_rhs.f90:1240-1245; BSSN adds nothing).
-template <typename A, bool Z4C, typename FX, typename FY, typename FZ>
-__device__ __forceinline__ A ko_term(const FX& X, const FY& Y, const FZ& Z, A add, const Coef<A>& C) {
-  if constexpr (Z4C && sizeof(A) == 8) {
-    auto x = [&](int o) { return __dadd_rn(X(o), add); };
-    auto y = [&](int o) { return __dadd_rn(Y(o), add); };
-    auto z = [&](int o) { return __dadd_rn(Z(o), add); };
-    return kodiv(ko_sum_rn<A, false>(x), C, 0) + kodiv(ko_sum_rn<A, false>(y), C, 1) + kodiv(ko_sum_rn<A, false>(z), C, 2);
-  } else {
-    return kodiv(ko_sum_rn<A, false>(X), C, 0) + kodiv(ko_sum_rn<A, false>(Y), C, 1) + kodiv(ko_sum_rn<A, false>(Z), C, 2);
-  }
+// KO dissipation of a point from its three lines.
+template <typename A, typename FX, typename FY, typename FZ>
+__device__ __forceinline__ A ko_term(const FX& X, const FY& Y, const FZ& Z, const Coef<A>& C) {
+  return kodiv(ko_sum_rn<A, false>(X), C, 0) + kodiv(ko_sum_rn<A, false>(Y), C, 1) + kodiv(ko_sum_rn<A, false>(Z), C, 2);
 }
 
 // March one field of one tile.  A: stencil arithmetic type, S: type of the
@@ -274,16 +274,17 @@ __device__ __forceinline__ A ko_term(const FX& X, const FY& Y, const FZ& Z, A ad
 // of the D array.
 template <typename A, int KIND, bool Z4C, typename T, typename S, typename SI>
 __device__ __forceinline__ void deriv_march(const StepBlock<T>& B, const S* src, const SI* in, const double* bsh,
-                                            int F, const DerivItem& it, T* D, int slots, int region,
+                                            int F, const DerivItem& it, T* D, int slots, int region, int spare,
                                             unsigned char* smem) {
   const Coef<A>& C = *reinterpret_cast<const Coef<A>*>(smem + kDerivCoef);
   if (threadIdx.x < sizeof(Coef<A>) / 4)
     reinterpret_cast<unsigned*>(smem + kDerivCoef)[threadIdx.x] = reinterpret_cast<const unsigned*>(&pick<A>(B.C))[threadIdx.x];
   A* ring = reinterpret_cast<A*>(smem);
   S* land = reinterpret_cast<S*>(smem + (size_t)DRING * DPLANE * sizeof(A));   // two planes, where A != S
-  // the thread's shift values, component c of point a of plane k at
-  // ((k % DBETA) * 6 + 2 c + a) * DTHREADS
-  double* bet = reinterpret_cast<double*>(smem + kDerivRing) + threadIdx.x;
+  // the thread's shift values, component c of point a in slot s at
+  // (6 s + 2 c + a) * DTHREADS
+  const double* bet = reinterpret_cast<double*>(smem + kDerivRing) + threadIdx.x;
+  const unsigned bet_s = (unsigned)__cvta_generic_to_shared(bet);
   const int ex0 = B.b.ex[0], ex1 = B.b.ex[1], ex2 = B.b.ex[2];
   const int x0 = it.x0, y0 = it.y0, k0 = it.k0, k1 = it.k1, W = it.w, NP = it.h / 2;
   const long long fs = B.b.fs;
@@ -319,9 +320,14 @@ __device__ __forceinline__ void deriv_march(const StepBlock<T>& B, const S* src,
   const int rx = region < 0 ? 0 : B.rlo[region][0], ry = region < 0 ? 0 : B.rlo[region][1];
   const int rz = region < 0 ? 0 : B.rlo[region][2];
   const int og = dl::g(F) * kDTile, oh = dl::h(F) * kDTile, oa = dl::a(F) * kDTile;
-  auto dptr = [&](int a, int k) -> T* {
-    const int dq = (i - rx) + rn0 * ((j + a - ry) + rn1 * (k - rz));
-    return D + ((long long)(B.dtile + (dq >> 7)) * (slots * kDTile) + (dq & 127));
+  const int rn01 = rn0 * rn1, dt0 = B.dtile;   // locals: the march's waits would have B read again each time
+  int dq = (i - rx) + rn0 * ((j - ry) + rn1 * (k0 - 2 - rz));   // entry of the first point at plane k
+  // a thread without a point of its own stores into the tile past the last
+  // (spare): straight-line code instead of a branch per point
+  T* const sp = D + (long long)spare * (slots * kDTile) + (threadIdx.x & 127);
+  auto dptr = [&](bool m, int q) -> T* {
+    T* d = D + ((long long)(dt0 + (q >> 7)) * (slots * kDTile) + (q & 127));
+    return m ? d : sp;
   };
   static_assert(kDTile == 128, "dptr");
 
@@ -337,17 +343,16 @@ __device__ __forceinline__ void deriv_march(const StepBlock<T>& B, const S* src,
 #pragma unroll
   for (int t = 0; t < 5; ++t) wx0[t] = wy0[t] = wx1[t] = wy1[t] = A(0);
 
-  // the shift at the points of plane k, from the stage input (bsh: its FP64
-  // side slots in the mixed form), copied two planes ahead
-  auto shift = [&](int k) {
-    if (k < k0 || k >= k1) return;
-    const double* b = sizeof(SI) == 4 ? bsh : (const double*)in + F_BETAX * fs;
-    const double* g = b + i + (long long)j * ex0 + (long long)k * P.sz;
-    double* s = bet + (k % DBETA) * 6 * DTHREADS;
+  // the shift at the points of plane k + 2, from the stage input (bsh: its FP64
+  // side slots in the mixed form), copied two planes ahead into slot sw
+  const double* gb = (sizeof(SI) == 4 ? bsh : (const double*)in + F_BETAX * fs) + i + (long long)j * ex0 +
+                     (long long)k0 * P.sz;
+  auto shift = [&](int sw) {
+    const unsigned s = bet_s + sw * (6 * DTHREADS * 8);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      if (m0) cp_async8(s + 2 * c * DTHREADS, g + c * fs, true);
-      if (m1) cp_async8(s + (2 * c + 1) * DTHREADS, g + c * fs + ex0, true);
+      if (m0) cp_async8(s + 2 * c * DTHREADS * 8, gb + c * fs);
+      if (m1) cp_async8(s + (2 * c + 1) * DTHREADS * 8, gb + c * fs + ex0);
     }
   };
 
@@ -390,18 +395,22 @@ __device__ __forceinline__ void deriv_march(const StepBlock<T>& B, const S* src,
 #pragma unroll
   for (int m = 0; m < DRING; ++m) so[m] = ((m + DRING - 3) % DRING) * DPLANE;
 #pragma unroll 1
-  for (int k = kA; k < kE; ++k) {
+  for (int k = kA, br = 0; k < kE; ++k) {
+    const int bw = br == 0 ? 2 : br - 1;         // the shift's slots of planes k (br) and k + 2
     const int par = (k - kA + 5) & 1;            // landing buffer of k+5
     P.issue(k + 5, ring + so[8], land + par * (DPER * DTHREADS));
-    shift(k + 2);
+    if (k + 2 >= k0 && k + 2 < k1) {
+      shift(bw);
+      gb += P.sz;
+    }
     cp_async_commit();
     const A* q = ring + so[3] + own;
     const bool outp = k >= k0 && k < k1 && !((fm & 4) && k == ex2 - 1) && !((fm & 32) && k == 0);
     if (any && outp) {
       const int fz = fits_z(k), cz = lop_codes(k, loz, ex2 - 1);
       const int f0 = fit0 & fz, f1 = fit1 & fz;
-      T* d0 = dptr(0, k);
-      T* d1 = dptr(1, k);
+      T* d0 = dptr(m0, dq);
+      T* d1 = dptr(m1, dq + rn0);
       A X0[7], X1[7], Y[8];   // x-lines of the two points; the y-line from row -3 to row 4
 #pragma unroll
       for (int o = -3; o <= 3; ++o)
@@ -432,55 +441,58 @@ __device__ __forceinline__ void deriv_march(const StepBlock<T>& B, const S* src,
         auto dd = [&](A fm2, A fm1, A f0, A f1, A f2, A cf) {
           return cf * (-fm2 + A(16) * fm1 - A(30) * f0 - f2 + A(16) * f1);
         };
-        if (m0) {
-          dstore(d0 + og, (T)wx0[4]);
-          dstore(d0 + og + kDTile, (T)wy0[4]);
-          dstore(d0 + oh, (T)dd(X0[1], X0[2], X0[3], X0[4], X0[5], C.Fdd[0]));
-          dstore(d0 + oh + 1 * kDTile, (T)(C.Fxy * (ds[0] - F8 * ds[1] + F8 * ds[3] - ds[4])));
-          dstore(d0 + oh + 3 * kDTile, (T)dd(Y[1], Y[2], Y[3], Y[4], Y[5], C.Fdd[1]));
-          dstore(d0 + oh + 5 * kDTile, (T)dd(c0[1], c0[2], c0[3], c0[4], c0[5], C.Fdd[2]));
-        }
-        if (m1) {
-          dstore(d1 + og, (T)wx1[4]);
-          dstore(d1 + og + kDTile, (T)wy1[4]);
-          dstore(d1 + oh, (T)dd(X1[1], X1[2], X1[3], X1[4], X1[5], C.Fdd[0]));
-          dstore(d1 + oh + 1 * kDTile, (T)(C.Fxy * (ds[1] - F8 * ds[2] + F8 * ds[4] - ds[5])));
-          dstore(d1 + oh + 3 * kDTile, (T)dd(Y[2], Y[3], Y[4], Y[5], Y[6], C.Fdd[1]));
-          dstore(d1 + oh + 5 * kDTile, (T)dd(c1[1], c1[2], c1[3], c1[4], c1[5], C.Fdd[2]));
-        }
+        dstore(d0 + og, (T)wx0[4]);
+        dstore(d0 + og + kDTile, (T)wy0[4]);
+        dstore(d0 + oh, (T)dd(X0[1], X0[2], X0[3], X0[4], X0[5], C.Fdd[0]));
+        dstore(d0 + oh + 1 * kDTile, (T)(C.Fxy * (ds[0] - F8 * ds[1] + F8 * ds[3] - ds[4])));
+        dstore(d0 + oh + 3 * kDTile, (T)dd(Y[1], Y[2], Y[3], Y[4], Y[5], C.Fdd[1]));
+        dstore(d0 + oh + 5 * kDTile, (T)dd(c0[1], c0[2], c0[3], c0[4], c0[5], C.Fdd[2]));
+        dstore(d1 + og, (T)wx1[4]);
+        dstore(d1 + og + kDTile, (T)wy1[4]);
+        dstore(d1 + oh, (T)dd(X1[1], X1[2], X1[3], X1[4], X1[5], C.Fdd[0]));
+        dstore(d1 + oh + 1 * kDTile, (T)(C.Fxy * (ds[1] - F8 * ds[2] + F8 * ds[4] - ds[5])));
+        dstore(d1 + oh + 3 * kDTile, (T)dd(Y[2], Y[3], Y[4], Y[5], Y[6], C.Fdd[1]));
+        dstore(d1 + oh + 5 * kDTile, (T)dd(c1[1], c1[2], c1[3], c1[4], c1[5], C.Fdd[2]));
       }
       if constexpr (KIND == 1) {
-        if (m0) {
-          dstore(d0 + og, (T)(C.d12[0] * (X0[1] - F8 * X0[2] + F8 * X0[4] - X0[5])));
-          dstore(d0 + og + kDTile, (T)(C.d12[1] * (Y[1] - F8 * Y[2] + F8 * Y[4] - Y[5])));
-        }
-        if (m1) {
-          dstore(d1 + og, (T)(C.d12[0] * (X1[1] - F8 * X1[2] + F8 * X1[4] - X1[5])));
-          dstore(d1 + og + kDTile, (T)(C.d12[1] * (Y[2] - F8 * Y[3] + F8 * Y[5] - Y[6])));
-        }
+        dstore(d0 + og, (T)(C.d12[0] * (X0[1] - F8 * X0[2] + F8 * X0[4] - X0[5])));
+        dstore(d0 + og + kDTile, (T)(C.d12[1] * (Y[1] - F8 * Y[2] + F8 * Y[4] - Y[5])));
+        dstore(d1 + og, (T)(C.d12[0] * (X1[1] - F8 * X1[2] + F8 * X1[4] - X1[5])));
+        dstore(d1 + og + kDTile, (T)(C.d12[1] * (Y[2] - F8 * Y[3] + F8 * Y[5] - Y[6])));
       }
       if constexpr (KIND <= 1) {
-        if (m0) dstore(d0 + og + 2 * kDTile, (T)(C.d12[2] * (c0[1] - F8 * c0[2] + F8 * c0[4] - c0[5])));
-        if (m1) dstore(d1 + og + 2 * kDTile, (T)(C.d12[2] * (c1[1] - F8 * c1[2] + F8 * c1[4] - c1[5])));
+        dstore(d0 + og + 2 * kDTile, (T)(C.d12[2] * (c0[1] - F8 * c0[2] + F8 * c0[4] - c0[5])));
+        dstore(d1 + og + 2 * kDTile, (T)(C.d12[2] * (c1[1] - F8 * c1[2] + F8 * c1[4] - c1[5])));
+      }
+      // FP64 advects the diagonal metric as g = d + 1; Z4c dissipates it so too
+      // (Z4c_rhs.f90:1240-1245), so there the lines are shifted once for both
+      constexpr bool kMetric = KIND == 0 && sizeof(A) == 8;
+      if constexpr (kMetric && Z4C) {
+#pragma unroll
+        for (int m = 0; m < 7; ++m) { X0[m] = X0[m] + add1; X1[m] = X1[m] + add1; }
+#pragma unroll
+        for (int m = 0; m < 8; ++m) Y[m] = Y[m] + add1;
+#pragma unroll
+        for (int m = 0; m < 7; ++m) { c0[m] = c0[m] + add1; c1[m] = c1[m] + add1; }
       }
       auto adv = [&](const auto& fX, const auto& fY, const auto& fZ, int a, int cy, int fit) -> A {
-        const double* sb = bet + ((k % DBETA) * 6 + a) * DTHREADS;
+        const double* sb = bet + (6 * br + a) * DTHREADS;
         auto line = [&](const auto& f, int d, int codes) {
           const A bv = (A)(T)sb[2 * d * DTHREADS];   // rounded as the pointwise pass sees it
           const A bd = bv * C.d12[d];
-          if constexpr (KIND == 0 && sizeof(A) == 8) return lop_term<A>([&](int o) { return f(o) + add1; }, bv, bd, codes);
+          if constexpr (kMetric && !Z4C) return lop_term<A>([&](int o) { return f(o) + add1; }, bv, bd, codes);
           else return lop_term<A>(f, bv, bd, codes);
         };
         const A r = line(fX, 0, cx) + line(fY, 1, cy) + line(fZ, 2, cz);
-        const A ko = C.ko * ko_term<A, Z4C && KIND == 0>(fX, fY, fZ, add1, C);
+        const A ko = C.ko * ko_term<A>(fX, fY, fZ, C);
         return ((fit & 8) ? r : A(0)) + ((fit & 4) ? ko : A(0));
       };
       const A a0 = adv([&](int o) { return X0[3 + o]; }, [&](int o) { return Y[3 + o]; },
                        [&](int o) { return c0[3 + o]; }, 0, cy0, f0);
-      if (m0) dstore(d0 + oa, (T)a0);
+      dstore(d0 + oa, (T)a0);
       const A a1 = adv([&](int o) { return X1[3 + o]; }, [&](int o) { return Y[4 + o]; },
                        [&](int o) { return c1[3 + o]; }, 1, cy1, f1);
-      if (m1) dstore(d1 + oa, (T)a1);
+      dstore(d1 + oa, (T)a1);
       if constexpr (KIND <= 1) {
         // next to an edge the derivatives are of 2nd order, on it zero.  One
         // copy of the code for both points
@@ -521,17 +533,13 @@ __device__ __forceinline__ void deriv_march(const StepBlock<T>& B, const S* src,
       // the mixed xz, yz derivatives of plane k-2 where they are of 4th order
       const int kl = k - 2;
       if (kl >= k0 && !((fm & 4) && kl == ex2 - 1) && !((fm & 32) && kl == 0)) {
-        const int fz = fits_z(kl);
-        if (m0 && (fit0 & fz & 1)) {
-          T* d = dptr(0, kl) + oh;
-          dstore(d + 2 * kDTile, (T)(C.d12[2] * (wx0[0] - F8 * wx0[1] + F8 * wx0[3] - wx0[4])));
-          dstore(d + 4 * kDTile, (T)(C.d12[2] * (wy0[0] - F8 * wy0[1] + F8 * wy0[3] - wy0[4])));
-        }
-        if (m1 && (fit1 & fz & 1)) {
-          T* d = dptr(1, kl) + oh;
-          dstore(d + 2 * kDTile, (T)(C.d12[2] * (wx1[0] - F8 * wx1[1] + F8 * wx1[3] - wx1[4])));
-          dstore(d + 4 * kDTile, (T)(C.d12[2] * (wy1[0] - F8 * wy1[1] + F8 * wy1[3] - wy1[4])));
-        }
+        const int fl = fits_z(kl);
+        T* d0 = dptr(m0 && (fit0 & fl & 1), dq - 2 * rn01) + oh;
+        T* d1 = dptr(m1 && (fit1 & fl & 1), dq - 2 * rn01 + rn0) + oh;
+        dstore(d0 + 2 * kDTile, (T)(C.d12[2] * (wx0[0] - F8 * wx0[1] + F8 * wx0[3] - wx0[4])));
+        dstore(d0 + 4 * kDTile, (T)(C.d12[2] * (wy0[0] - F8 * wy0[1] + F8 * wy0[3] - wy0[4])));
+        dstore(d1 + 2 * kDTile, (T)(C.d12[2] * (wx1[0] - F8 * wx1[1] + F8 * wx1[3] - wx1[4])));
+        dstore(d1 + 4 * kDTile, (T)(C.d12[2] * (wy1[0] - F8 * wy1[1] + F8 * wy1[3] - wy1[4])));
       }
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
@@ -547,6 +555,8 @@ __device__ __forceinline__ void deriv_march(const StepBlock<T>& B, const S* src,
 #pragma unroll
     for (int m = 0; m < DRING - 1; ++m) so[m] = so[m + 1];
     so[DRING - 1] = s0;
+    dq += rn01;
+    br = br == 2 ? 0 : br + 1;
   }
   cp_async_wait<0>();   // the copies still in flight land before the ring is reused
 }
@@ -559,7 +569,7 @@ __device__ __forceinline__ void deriv_march(const StepBlock<T>& B, const S* src,
 template <typename T, typename SI, bool Z4C>
 __global__ void __launch_bounds__(DTHREADS, AMSS_DMINB) k_deriv(const StepBlock<T>* __restrict__ blocks,
                                                        const DerivItem* __restrict__ items, int nitems, int sub,
-                                                       T* __restrict__ D, int slots, int region) {
+                                                       T* __restrict__ D, int slots, int region, int spare) {
   extern __shared__ __align__(16) unsigned char smem[];
   for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
     const DerivItem it = items[w];
@@ -575,31 +585,32 @@ __global__ void __launch_bounds__(DTHREADS, AMSS_DMINB) k_deriv(const StepBlock<
         // wide fields of the mixed form: FP64 source (state, or the FP64 side stage) and arithmetic
         const double* src = sizeof(SI) == 4 ? B.side[sub == 2 ? 1 : 0] + side_slot(F) * fs
                                             : (const double*)in + F * fs;
-        deriv_march<double, 0, Z4C>(B, src, in, bsh, F, it, D, slots, region, smem);
+        deriv_march<double, 0, Z4C>(B, src, in, bsh, F, it, D, slots, region, spare, smem);
         __syncthreads();
         continue;
       }
     }
     const SI* src = in + F * fs;
     switch (dkind(F)) {
-      case 0: deriv_march<T, 0, Z4C>(B, src, in, bsh, F, it, D, slots, region, smem); break;
-      case 1: deriv_march<T, 1, Z4C>(B, src, in, bsh, F, it, D, slots, region, smem); break;
-      default: deriv_march<T, 2, Z4C>(B, src, in, bsh, F, it, D, slots, region, smem); break;
+      case 0: deriv_march<T, 0, Z4C>(B, src, in, bsh, F, it, D, slots, region, spare, smem); break;
+      case 1: deriv_march<T, 1, Z4C>(B, src, in, bsh, F, it, D, slots, region, spare, smem); break;
+      default: deriv_march<T, 2, Z4C>(B, src, in, bsh, F, it, D, slots, region, spare, smem); break;
     }
     __syncthreads();
   }
 }
 
 // Stencil pass launcher: substep 0 reads the FP64 state, 1-3 the stages;
-// region: the D order of the points (-1: whole arrays, else StepBlock::rlo).
+// region: the D order of the points (-1: whole arrays, else StepBlock::rlo);
+// spare: a tile of D that holds no points (any rubbish may be stored there).
 template <typename T, typename SS>
 cudaError_t launch_deriv(const void* blocks, const DerivItem* items, int nitems, int sub, void* D, int slots,
-                         int region, int grid, cudaStream_t s) {
+                         int region, int spare, int grid, cudaStream_t s) {
   const StepBlock<T>* bl = (const StepBlock<T>*)blocks;
   auto go = [&](auto kernel) -> cudaError_t {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDerivSmem);
     if (e != cudaSuccess) return e;
-    kernel<<<grid, DTHREADS, kDerivSmem, s>>>(bl, items, nitems, sub, (T*)D, slots, region);
+    kernel<<<grid, DTHREADS, kDerivSmem, s>>>(bl, items, nitems, sub, (T*)D, slots, region, spare);
     return cudaGetLastError();
   };
   if (slots == D_SLOTS_Z4C) return sub == 0 ? go(k_deriv<T, double, true>) : go(k_deriv<T, SS, true>);

@@ -2,5 +2,6 @@
 #include "deriv.cuh"
 
 namespace amss {
-template cudaError_t launch_deriv<float, float>(const void*, const DerivItem*, int, int, void*, int, int, int, cudaStream_t);
+template cudaError_t launch_deriv<float, float>(const void*, const DerivItem*, int, int, void*, int, int, int, int,
+                                             cudaStream_t);
 }  // namespace amss

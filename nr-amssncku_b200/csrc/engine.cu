@@ -41,7 +41,7 @@ cudaError_t launch_face(const void* blocks, const int2* faces, int nfaces, int s
                         unsigned* status, cudaStream_t s);
 template <typename T, typename SS>
 cudaError_t launch_deriv(const void* blocks, const DerivItem* items, int nitems, int sub, void* D, int slots,
-                         int region, int grid, cudaStream_t s);
+                         int region, int spare, int grid, cudaStream_t s);
 cudaError_t launch_enforce(long long n, long long fs, double* g, double* a, cudaStream_t s);
 template <typename T>
 cudaError_t launch_constraints(const void* table, const int2* tiles, int ntiles, int tile_pts, bool symm,
@@ -585,6 +585,7 @@ extern "C" int amss_engine_commit(amss_engine* e) {
   if (e->prm.kernel == 0) {
     long long mx = 0;
     for (auto& kv : e->levels) mx = std::max(mx, (long long)kv.second.dtiles_n * kDTile);
+    if (mx) mx += kDTile;   // the stencil pass's spare tile
     const int slots = e->nf == NFIELDS_Z4C ? D_SLOTS_Z4C : D_SLOTS;
     if (mx) AMSS_CK(cudaMalloc(&e->D, (size_t)mx * slots * (mixed ? sizeof(float) : sizeof(double))));
   }
@@ -789,8 +790,8 @@ static int step_level_impl(amss_engine* e, int level, double dt, bool fin = fals
     if (split && nditems) {
       const int slots = e->nf == NFIELDS_Z4C ? D_SLOTS_Z4C : D_SLOTS, region = reg ? 0 : own ? 1 : -1;
       const cudaError_t ed =
-          mixed ? launch_deriv<float, float>(L.dtable, ditems, nditems, sub, e->D, slots, region, dgrid, e->stream)
-                : launch_deriv<double, double>(L.dtable, ditems, nditems, sub, e->D, slots, region, dgrid, e->stream);
+          mixed ? launch_deriv<float, float>(L.dtable, ditems, nditems, sub, e->D, slots, region, L.dtiles_n, dgrid, e->stream)
+                : launch_deriv<double, double>(L.dtable, ditems, nditems, sub, e->D, slots, region, L.dtiles_n, dgrid, e->stream);
       AMSS_CK(ed);
       e->launches++;
     }
