@@ -43,15 +43,20 @@ enum StatusBits : unsigned {
   ST_TIMEOUT = 16u,   // a bounded wait on an asynchronous copy gave up
 };
 
-// Parity of each state field under reflection x, y, z (bssn_class.C:177-330).
+// Parity of each state field under reflection x, y, z (bssn_class.C:177-330):
+// bit F of antisym(dir) set = field F antisymmetric in that direction.  One
+// word a direction: a table indexed by a field known at run time only would be
+// built on the stack at every use.
+__host__ __device__ constexpr unsigned antisym(int dir) {
+  // bits x, y, z of chi trK gxx gxy gxz gyy gyz gzz | Axx .. Azz | Gam Lap beta | dtSf TZ
+  constexpr unsigned char anti[25] = {0, 0, 0, 3, 5, 0, 6, 0, 0, 3, 5, 0, 6, 0, 1, 2, 4, 0, 1, 2, 4, 1, 2, 4, 0};
+  unsigned m = 0;
+  for (int f = 0; f < 25; ++f) m |= (unsigned)((anti[f] >> dir) & 1) << f;
+  return m;
+}
 __host__ __device__ constexpr int soa_sign(int field, int dir) {
-  // bit set = antisymmetric in that direction
-  constexpr unsigned char anti[25] = {
-      0, 0, 0, 3, 5, 0, 6, 0,   // chi trK gxx gxy gxz gyy gyz gzz
-      0, 3, 5, 0, 6, 0,         // Axx .. Azz
-      1, 2, 4, 0, 1, 2, 4,      // Gamx Gamy Gamz Lap betax betay betaz
-      1, 2, 4, 0};              // dtSfx dtSfy dtSfz TZ
-  return (anti[field] >> dir) & 1 ? -1 : 1;
+  constexpr unsigned m[3] = {antisym(0), antisym(1), antisym(2)};
+  return ((dir == 0 ? m[0] : dir == 1 ? m[1] : m[2]) >> field) & 1u ? -1 : 1;
 }
 
 // One block as the kernels see it.

@@ -13,7 +13,7 @@ namespace amss {
 // a field, and the points of an x face share no line -- so the fields of a
 // point go to different warps and their loads are in flight together: 82 us a
 // launch on a 70^3 block (28,568 face points) and 93 us on a 24^3 block with
-// one thread taking the 24 fields of a point in turn, 36 us and 12 us
+// one thread taking the 24 fields of a point in turn, 30 us and 10 us
 // now.  enforce_ga couples 12 fields of a point, which meet in shared memory;
 // warp 0 then finishes one point per lane.
 constexpr int kFacePts = 32;
