@@ -21,6 +21,21 @@ __device__ __forceinline__ bool amr_inside(const AmrBlock& b, int gi, int gj, in
 }
 __device__ __forceinline__ double* amr_state(const AmrBlock& b) { return b.tl[b.lvl[0]]; }
 
+// Copies the n fields of one point: eight loads in flight before their stores
+// (the compiler may not move a load past a store it cannot tell apart).
+template <typename V>
+__device__ __forceinline__ void copy_point(V* d, const V* s, long long dfs, long long sfs, int n) {
+  for (int f0 = 0; f0 < n; f0 += 8) {
+    V v[8];
+#pragma unroll
+    for (int f = 0; f < 8; ++f)
+      if (f0 + f < n) v[f] = s[(f0 + f) * sfs];
+#pragma unroll
+    for (int f = 0; f < 8; ++f)
+      if (f0 + f < n) d[(f0 + f) * dfs] = v[f];
+  }
+}
+
 // Same-level ghost fill: copy the nf fields of each box point from src to dst.
 template <typename SS>
 __global__ void k_amr_sync(const AmrBlock* __restrict__ blocks, const AmrBox* __restrict__ boxes,
@@ -39,15 +54,13 @@ __global__ void k_amr_sync(const AmrBlock* __restrict__ blocks, const AmrBox* __
     if (which == BUF_STATE || which == BUF_TEMP) {
       const double* s = which == BUF_STATE ? amr_state(S) : S.K;
       double* d = which == BUF_STATE ? amr_state(D) : D.K;
-      for (int f = 0; f < D.nf; ++f) d[f * D.fs + od] = s[f * S.fs + os];
+      copy_point(d + od, s + os, D.fs, S.fs, D.nf);
     } else {
       const int sl = which == BUF_STAGE_A ? 0 : 1;
       const SS* s = (const SS*)S.st[sl];
       SS* d = (SS*)D.st[sl];
-      for (int f = 0; f < D.nf; ++f) d[f * D.fs + od] = s[f * S.fs + os];
-      if constexpr (sizeof(SS) == 4) {
-        for (int f = 0; f < kSideFields; ++f) D.side[sl][f * D.fs + od] = S.side[sl][f * S.fs + os];
-      }
+      copy_point(d + od, s + os, D.fs, S.fs, D.nf);
+      if constexpr (sizeof(SS) == 4) copy_point(D.side[sl] + od, (const double*)S.side[sl] + os, D.fs, S.fs, kSideFields);
     }
   }
 }
@@ -231,17 +244,25 @@ __device__ __forceinline__ void timeinterp_point(const AmrBlock& B, long long p)
   const double* f1 = B.tl[cur];
   const double* f2 = B.tl[(cur + 2) % 3];
   const double* f3 = B.tl[(cur + 1) % 3];
-  if (B.lvl[1] >= 2) {
-    const double C1 = 3.0 / 8.0, C2 = 3.0 / 4.0, C3 = -1.0 / 8.0;
-    for (int f = 0; f < B.nf; ++f) {
-      const long long o = f * B.fs + p;
-      B.K[o] = __dadd_rn(__dadd_rn(__dmul_rn(C1, f1[o]), __dmul_rn(C2, f2[o])), __dmul_rn(C3, f3[o]));
-    }
-  } else {
-    for (int f = 0; f < B.nf; ++f) {
-      const long long o = f * B.fs + p;
-      B.K[o] = __dmul_rn(0.5, __dadd_rn(f1[o], f2[o]));
-    }
+  const bool second = B.lvl[1] >= 2;
+  const double C1 = 3.0 / 8.0, C2 = 3.0 / 4.0, C3 = -1.0 / 8.0;
+  // four fields' loads in flight before their stores
+  for (int f0 = 0; f0 < B.nf; f0 += 4) {
+    double v1[4], v2[4], v3[4];
+#pragma unroll
+    for (int f = 0; f < 4; ++f)
+      if (f0 + f < B.nf) {
+        const long long o = (f0 + f) * B.fs + p;
+        v1[f] = f1[o];
+        v2[f] = f2[o];
+        v3[f] = second ? f3[o] : 0.0;
+      }
+#pragma unroll
+    for (int f = 0; f < 4; ++f)
+      if (f0 + f < B.nf)
+        B.K[(f0 + f) * B.fs + p] =
+            second ? __dadd_rn(__dadd_rn(__dmul_rn(C1, v1[f]), __dmul_rn(C2, v2[f])), __dmul_rn(C3, v3[f]))
+                   : __dmul_rn(0.5, __dadd_rn(v1[f], v2[f]));
   }
 }
 
