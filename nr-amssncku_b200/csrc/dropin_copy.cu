@@ -13,8 +13,8 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <exception>
 #include <new>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -121,7 +121,7 @@ cudaError_t copy_fields(CopyPool& P, const CopyField* fields, int nfields, size_
     try {
       for (int w = 1; w < nw; ++w)
         t.emplace_back([&, w] { work(P, w, v, next, to_device, err); });
-    } catch (const std::system_error&) {   // no more threads: the ones there are, and this one, do it
+    } catch (const std::exception&) {   // no more threads, or no memory for one: those there are, and this one, do it
     }
     work(P, 0, v, next, to_device, err);
     for (std::thread& x : t) x.join();
