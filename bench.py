@@ -345,7 +345,7 @@ def run_ours(args, rank, world):
         "clocks": r["clocks"],
         "nan": r["nan"],
         "tiling": {"per_level": r["tiling"], "what": "stencil-pass tile width (0 = default), z-slabs per block, "
-                                                    "occupancy form (0: 2 CTAs/SM, 1: 4 FP64 / 3 FP32) and the "
+                                                    "occupancy setting (one compiled form: 0) and the "
                                                     "tuner's ms per level step, chosen by amss_b200.autotune before "
                                                     "the timed region"},
         "punctures_after_warmup_and_timed_steps": r["tracked"],
@@ -611,7 +611,7 @@ def main():
     ap.add_argument("--tune", type=int, default=1, help="pick each level's stencil-pass tiling with the autotuner")
     ap.add_argument("--tune-cache", default="", help="JSON cache of tuned tilings (default: none, tune every run)")
     ap.add_argument("--occupancy", type=int, choices=[0, 1], default=None,
-                    help="with --tune 0: the stencil pass's occupancy form on every level (default: the engine's, 0)")
+                    help="with --tune 0: the occupancy setting of every level (recorded only: one compiled form)")
     ap.add_argument("--no-parts", action="store_true",
                     help="FP64 line only: skip the mixed-form and adjoint parts of the metric")
     ap.add_argument("--report", choices=["none", "mixed"], default="none",

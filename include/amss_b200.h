@@ -280,17 +280,18 @@ int amss_engine_run_graph(amss_engine* e, int level, double dt, int nsteps, int 
 
 /* No counterpart in the reference (its work split is the MPI block layout).
  * Tiling of the stencil pass of one level, the knob amss_b200.autotune
- * searches: x-y tile width (8..64 columns, H = 256 / width rows; 0 restores
- * the default, the block's x extent cut into pieces of at most 64) and the
+ * searches: x-y tile width (8..64 columns, at most 38 used; 0 restores the
+ * default, the block's x extent cut into equal pieces of at most 38) and the
  * number of z-slabs each block's march is cut into (1..16; slabs are at least
- * 8 planes).  Results do not depend on it.  Waits for the engine's stream;
- * not inside a stream capture. */
+ * 8 planes).  0 and 1 together, the initial setting, let the engine choose the
+ * slabs.  Results do not depend on it.  Waits for the engine's stream; not
+ * inside a stream capture. */
 int amss_engine_set_level_tiling(amss_engine* e, int level, int tile_w, int zsplit);
 /* The level's tiling (as set; 0 = default width) and its stencil work items. */
 int amss_engine_get_level_tiling(amss_engine* e, int level, int* tile_w, int* zsplit, int* nitems);
-/* No reference counterpart: which compiled form of the stencil pass a level
- * uses, 0 (two resident CTAs per SM, the default) or 1 (four in FP64, three in
- * FP32, fewer registers with some spills).  Results do not depend on it. */
+/* No reference counterpart: a level's occupancy setting, 0 (the default) or 1.
+ * The stencil pass has one compiled form, two resident CTAs per SM, so the
+ * setting is recorded and returned and changes nothing else. */
 int amss_engine_set_level_occupancy(amss_engine* e, int level, int occ);
 int amss_engine_get_level_occupancy(amss_engine* e, int level, int* occ);
 /* No reference counterpart: the cells a coarse step's final RK4 substep

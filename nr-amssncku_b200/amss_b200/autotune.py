@@ -2,11 +2,9 @@
 
 The stencil pass (k_deriv) runs one CTA per (field, x-y tile, z-slab) work
 item.  How its items fill the GPU depends on each level's block shapes: the
-tile width W (H = 256 / W rows) sets the halo overhead and the item count, the
-z-split trades a 7-plane prologue per slab for more, shorter items that fill
-the last wave of CTAs better, and the occupancy form (two resident CTAs per SM,
-or four in FP64 / three in FP32 with fewer registers and some spills) trades
-spills for warps.  The tuner times each
+tile width W sets the halo overhead and the item count, and the z-split trades a
+prologue of planes per slab for more, shorter items that fill the last wave of
+CTAs better; (0, 1) stands for the engine's own choice.  The tuner times each
 candidate on a scratch engine holding the same hierarchy and state (CUDA
 events around graph replays of that level's RK4 step; the live engine is not
 touched), keeps the fastest per level, and caches the choice in a JSON file
@@ -26,23 +24,24 @@ DEFAULT_CACHE = os.path.join(os.path.expanduser("~"), ".cache", "amss_b200", "ti
 
 def level_key(H, level, precision, formulation):
     shapes = sorted(tuple(H.blocks[i].ex) for p in H.levels[level] for i in p.blocks)
-    return f"{precision}/{formulation}/" + ";".join("x".join(map(str, s)) for s in shapes)
+    # tile38: the stencil pass's widest tile; times of passes with other tiles don't carry over
+    return f"{precision}/{formulation}/tile38/" + ";".join("x".join(map(str, s)) for s in shapes)
 
 
 def candidates(H, level):
     """(tile width, z-split, occupancy) worth timing for a level: the default
     width and the widths that cut the level's smallest block width into 1-3
-    near-equal tiles, each with 1-4 z-slabs, in both occupancy forms."""
+    near-equal tiles, each with 1-4 z-slabs (occupancy 0: one compiled form)."""
     wmin = min(H.blocks[i].ex[0] for p in H.levels[level] for i in p.blocks)
     widths = {0}
     for parts in (1, 2, 3):
         w = -(-wmin // parts)
-        if 8 <= w <= 64:
+        if 8 <= w <= 38:
             widths.add(w)
     for w in (16, 32):
         if w <= wmin:
             widths.add(w)
-    return [(w, z, o) for w in sorted(widths) for z in (1, 2, 3, 4) for o in (0, 1)]
+    return [(w, z, o) for w in sorted(widths) for z in (1, 2, 3, 4) for o in (0,)]
 
 
 def _time_level(eng, level, dt, reps):

@@ -177,13 +177,14 @@ class Engine:
 
     def set_level_tiling(self, level, tile_w=0, zsplit=1):
         """Stencil-pass tiling of one level (amss_engine_set_level_tiling):
-        tile width 8..64 (0: default) and z-slabs per block."""
+        tile width 8..64, at most 38 used (0: default), and z-slabs per
+        block; (0, 1) lets the engine choose the slabs."""
         check(lib().amss_engine_set_level_tiling(self._h, level, int(tile_w), int(zsplit)),
               "amss_engine_set_level_tiling")
 
     def set_level_occupancy(self, level, occ):
-        """Compiled form of a level's stencil pass: 0 (two resident CTAs per
-        SM) or 1 (four in FP64, three in FP32)."""
+        """Occupancy setting of a level, 0 or 1: recorded only, as the stencil
+        pass has one compiled form."""
         check(lib().amss_engine_set_level_occupancy(self._h, level, int(occ)), "amss_engine_set_level_occupancy")
 
     def level_occupancy(self, level):

@@ -14,7 +14,7 @@
 // planes late, so that each is formed once.
 //
 // The pass is bound by instruction issue and latency, not by memory (417 MB in
-// 264 us on 70^3 points; of 9,000 instructions a point 2,100 are FP64), so the
+// 264 us on 70^3 points; at 291 us 2,100 of 10,200 thread instructions a point were FP64), so the
 // layout serves those: two columns a thread share the row differences of the
 // cross stencil, the y-line, and a step's barrier, gates and addresses; the
 // row stride is a constant, so that a stencil's reads differ by immediates;

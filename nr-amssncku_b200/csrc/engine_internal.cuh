@@ -139,7 +139,7 @@ struct ELevel {
   int nditems_s = 0;
   int tile_w = 0;               // stencil-pass tile width as set (0: default; at most DWMAX is used)
   int zsplit = 1;               // z-slabs per block in the stencil pass
-  int docc = 0;                 // stencil-pass occupancy form: 0 two resident CTAs, 1 more (deriv.cuh)
+  int docc = 0;                 // occupancy setting, recorded only (one compiled form)
   int dtiles_n = 0;             // D tiles of this level
   long long dfs = 0;            // field stride of the level's scratch arrays (constraints, Psi4)
   int* dregion = nullptr;       // per table block: local [lo, hi) of its owned cells inside its patch
