@@ -22,7 +22,9 @@ __device__ __forceinline__ bool amr_inside(const AmrBlock& b, int gi, int gj, in
 __device__ __forceinline__ double* amr_state(const AmrBlock& b) { return b.tl[b.lvl[0]]; }
 
 // Copies the n fields of one point: eight loads in flight before their stores
-// (the compiler may not move a load past a store it cannot tell apart).
+// (the compiler may not move a load past a store it cannot tell apart).  With
+// the time interpolation's batches below, the 7-level binary's coarse step
+// 276.7 -> 275.5 ms, mixed 206.7 -> 205.7 ms.
 template <typename V>
 __device__ __forceinline__ void copy_point(V* d, const V* s, long long dfs, long long sfs, int n) {
   for (int f0 = 0; f0 < n; f0 += 8) {

@@ -13,9 +13,10 @@
 // register windows of Dx f and Dy f at planes k-4 .. k, and are stored two
 // planes late, so that each is formed once.
 //
-// The pass is bound by instruction issue and latency, not by memory (417 MB in
-// 264 us on 70^3 points; at 291 us 2,100 of 10,200 thread instructions a point were FP64), so the
-// layout serves those: two columns a thread share the row differences of the
+// The pass is bound by instruction issue (43 % of the cycles) and latency, not
+// by memory (417 MB in 268 us on 70^3 points), and most of what it issues is
+// not arithmetic (2,100 of 10,200 thread instructions a point were FP64 in the
+// 291 us form below), so the layout serves those: two columns a thread share the row differences of the
 // cross stencil, the y-line, and a step's barrier, gates and addresses; the
 // row stride is a constant, so that a stencil's reads differ by immediates;
 // the shift comes through shared memory two planes ahead, the coefficients
@@ -117,9 +118,9 @@ inline void deriv_push(std::vector<DerivItem>& v, int block, const int lo[3], co
 // item of p planes takes p + 6 steps (four of warm-up, the prologue about two)
 // of relative cost 1, 0.65 or 0.5 by its field's kind; the launch takes the
 // longest item, or all items shared out plus part of a last one.  A 24^3 block
-// is 48 items of 30 steps uncut and 288 of 10 in six slabs (a step 512 and
-// 243 us); 70^3
-// points are best in two (2.01 ms a step; 2.33 uncut, 2.07 in three).
+// is 48 items of 30 steps uncut and 288 of 10 in six slabs (a step 459 and
+// 216 us); 70^3 points go in two (1.92 ms a step; 2.17 uncut, 1.94 in three,
+// 1.89 in four), 134^3 of Z4c in one or two alike (12.2 and 12.3 ms).
 inline int deriv_slabs(const std::vector<DerivItem>& one, bool z4c, int ctas) {
   const double per_tile = 11.0 + (z4c ? 5 : 4) * 0.65 + 9 * 0.5;
   int best = 1;
