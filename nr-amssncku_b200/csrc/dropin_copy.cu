@@ -102,8 +102,10 @@ void work(CopyPool& P, int w, const std::vector<Piece>& v, std::atomic<size_t>& 
 cudaError_t copy_fields(CopyPool& P, const CopyField* fields, int nfields, size_t bytes, bool to_device,
                         cudaStream_t s) try {
   const size_t total = bytes * nfields;
-  // below about 4 MB the threads cost more than they save
-  if (total >= ((size_t)4 << 20) && P.init()) {
+  // Starting the threads costs more than they save where the arrays' pages are
+  // there already: at 26^3 points (4.8 MB in, 7.7 MB out) 2.4 ms a call by
+  // plain copies, 2.7 to 3.1 ms by threads; at 28^3 (6.0 and 9.7 MB) 5.0 and 2.3.
+  if (total >= ((size_t)8 << 20) && P.init()) {
     // work of this context's stream that the copies must follow (outputs), or
     // that still reads the arrays they fill (inputs)
     cudaError_t e = cudaStreamSynchronize(s);

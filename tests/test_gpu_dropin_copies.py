@@ -1,5 +1,5 @@
 """The drop-in right-hand side on arrays large enough for the threaded copies
-(4 MB in all; fields of more than one 1 MB piece, with a remainder): against
+(8 MB in all; fields of more than one 1 MB piece, with a remainder): against
 the oracle, and from two threads at once, each with its own pool of pieces."""
 import threading
 
@@ -20,9 +20,9 @@ def _inputs(ex, seed):
 
 
 def test_smallest_threaded_call_equals_the_plain_copies():
-    """15,876 points, 4.1 MB in: the entry that allocates nothing runs the same
+    """30,996 points, 8.4 MB in: the entry that allocates nothing runs the same
     kernel over plain copies."""
-    X, st = _inputs((27, 28, 21), 3)
+    X, st = _inputs((27, 28, 41), 3)
     got = dropin.compute_rhs_bssn(*X, st, eps=0.1, co=0)
     ref = dropin.compute_rhs_bssn_noalloc(*X, st, eps=0.1, co=0)
     assert got[0] == ref[0] == 0
