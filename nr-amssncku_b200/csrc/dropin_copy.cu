@@ -127,6 +127,14 @@ cudaError_t copy_fields(CopyPool& P, const CopyField* fields, int nfields, size_
     }
     work(P, 0, v, next, to_device, err);
     for (std::thread& x : t) x.join();
+    if (err.load() != 0) {
+      // a worker stopped with copies in flight: they end before the caller's
+      // arrays, the device's and the pieces are used again.  Later calls take
+      // the plain copies.
+      for (int w = 0; w < kCopyWorkers; ++w) (void)cudaStreamSynchronize(P.stream[w]);
+      P.release();
+      P.failed = true;
+    }
     return (cudaError_t)err.load();
   }
   for (int m = 0; m < nfields; ++m) {

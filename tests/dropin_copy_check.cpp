@@ -1,0 +1,189 @@
+// Runs copy_fields (csrc/dropin_copy.cu, compiled as host C++) over a stand-in
+// for the CUDA runtime whose "device" is host memory and whose streams hold
+// their copies until something waits for them, so that what a call leaves in
+// flight can be counted and any runtime call can be made to fail.
+// usage: dropin_copy_check <scenario>; exit status 0: as it should be.
+#include <algorithm>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <map>
+#include <mutex>
+#include <set>
+#include <string>
+#include <vector>
+
+#include "dropin_ctx.cuh"
+
+namespace {
+
+struct Copy {
+  void* dst;
+  const void* src;
+  size_t n;
+};
+struct Stream {
+  std::vector<Copy> queued;
+};
+std::mutex mu;
+std::set<Stream*> streams;
+std::map<void*, Stream*> events;           // event -> stream it was recorded on
+std::vector<char*> pinned;                 // live pinned buffers
+int copies = 0, waits = 0;                 // calls so far
+int fail_copy = -1, fail_wait = -1;        // the call that fails, counted from 0
+int plain = 0, pieces = 0;                 // copies on the caller's stream, and on others
+Stream* caller = nullptr;
+
+void finish(Stream* s) {
+  for (const Copy& c : s->queued) std::memcpy(c.dst, c.src, c.n);
+  s->queued.clear();
+}
+size_t in_flight() {
+  size_t n = 0;
+  for (Stream* s : streams) n += s->queued.size();
+  return n;
+}
+Stream* of(cudaStream_t s) { return reinterpret_cast<Stream*>(s); }
+
+}  // namespace
+
+extern "C" {
+cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
+  std::lock_guard<std::mutex> g(mu);
+  pinned.push_back((char*)(*p = std::malloc(n)));
+  return cudaSuccess;
+}
+cudaError_t cudaFreeHost(void* p) {
+  std::lock_guard<std::mutex> g(mu);
+  pinned.erase(std::find(pinned.begin(), pinned.end(), (char*)p));
+  std::free(p);
+  return cudaSuccess;
+}
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
+  std::lock_guard<std::mutex> g(mu);
+  Stream* n = new Stream;
+  streams.insert(n);
+  *s = reinterpret_cast<cudaStream_t>(n);
+  return cudaSuccess;
+}
+cudaError_t cudaStreamDestroy(cudaStream_t s) {
+  std::lock_guard<std::mutex> g(mu);
+  finish(of(s));
+  streams.erase(of(s));
+  delete of(s);
+  return cudaSuccess;
+}
+cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+  std::lock_guard<std::mutex> g(mu);
+  finish(of(s));
+  return cudaSuccess;
+}
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
+  *e = reinterpret_cast<cudaEvent_t>(new char);
+  return cudaSuccess;
+}
+cudaError_t cudaEventDestroy(cudaEvent_t e) {
+  delete reinterpret_cast<char*>(e);
+  return cudaSuccess;
+}
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+  std::lock_guard<std::mutex> g(mu);
+  events[e] = of(s);
+  return cudaSuccess;
+}
+cudaError_t cudaEventSynchronize(cudaEvent_t e) {
+  std::lock_guard<std::mutex> g(mu);
+  if (waits++ == fail_wait) return cudaErrorUnknown;
+  finish(events[e]);
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind, cudaStream_t s) {
+  std::lock_guard<std::mutex> g(mu);
+  if (copies++ == fail_copy) return cudaErrorUnknown;
+  of(s)->queued.push_back(Copy{dst, src, n});
+  ++(of(s) == caller ? plain : pieces);
+  return cudaSuccess;
+}
+}
+
+using namespace amss;
+
+namespace {
+
+#define EXPECT(c)                                              \
+  do {                                                         \
+    if (!(c)) {                                                \
+      std::fprintf(stderr, "line %d: %s\n", __LINE__, #c);     \
+      std::exit(1);                                            \
+    }                                                          \
+  } while (0)
+
+constexpr int kFields = 12;
+constexpr size_t kBytes = (size_t)1300 * 1000;   // a piece and a remainder; 15.6 MB in all
+std::vector<std::vector<char>> host(kFields), dev(kFields);
+cudaStream_t stream;
+
+std::vector<CopyField> fields() {
+  std::vector<CopyField> f;
+  for (int m = 0; m < kFields; ++m) f.push_back(CopyField{dev[m].data(), host[m].data()});
+  return f;
+}
+void fill() {
+  for (int m = 0; m < kFields; ++m) {
+    host[m].assign(kBytes, 0);
+    dev[m].assign(kBytes, 0);
+    for (size_t i = 0; i < kBytes; ++i) {
+      host[m][i] = (char)(7 * m + i % 251);
+      dev[m][i] = (char)(5 * m + i % 241 + 1);
+    }
+  }
+}
+
+// A failed call leaves nothing in flight: its pinned pieces and the device
+// arrays may be reused at once.  The calls after it take the plain copies.
+void failed(int at_copy, int at_wait) {
+  for (const bool to_device : {true, false}) {
+    CopyPool pool;
+    fill();
+    copies = waits = 0;
+    fail_copy = at_copy;
+    fail_wait = at_wait;
+    EXPECT(copy_fields(pool, fields().data(), kFields, kBytes, to_device, stream) == cudaErrorUnknown);
+    EXPECT(in_flight() == 0);
+    fail_copy = fail_wait = -1;
+    fill();
+    plain = pieces = 0;
+    EXPECT(copy_fields(pool, fields().data(), kFields, kBytes, to_device, stream) == cudaSuccess);
+    cudaStreamSynchronize(stream);
+    EXPECT(plain == kFields && pieces == 0);
+    EXPECT(host == dev);
+  }
+}
+
+void works() {
+  for (const bool to_device : {true, false}) {
+    CopyPool pool;
+    fill();
+    plain = pieces = 0;
+    EXPECT(copy_fields(pool, fields().data(), kFields, kBytes, to_device, stream) == cudaSuccess);
+    EXPECT(in_flight() == 0 && plain == 0 && pieces == 2 * kFields);
+    EXPECT(host == dev);
+  }
+}
+
+}  // namespace
+
+int main(int, char** argv) {
+  cudaStreamCreateWithFlags(&stream, 0);
+  caller = of(stream);
+  const std::string s = argv[1];
+  if (s == "works") works();
+  else if (s == "copy_fails") failed(20, -1);
+  else if (s == "wait_fails") failed(-1, 5);
+  else return 2;
+  EXPECT(pinned.empty());   // given back with the pool
+  return 0;
+}
