@@ -26,7 +26,7 @@ struct CopyField {
   void* host;
 };
 // Copies `bytes` of every field host -> device or back.  In stream order with
-// s; the threaded form has also completed on return.
+// s; the copies that threads made have also completed on return.
 cudaError_t copy_fields(CopyPool& pool, const CopyField* fields, int nfields, size_t bytes, bool to_device,
                         cudaStream_t s);
 

@@ -33,6 +33,7 @@ int copies = 0, waits = 0;                 // calls so far
 int fail_copy = -1, fail_wait = -1;        // the call that fails, counted from 0
 int plain = 0, pieces = 0;                 // copies on the caller's stream, and on others
 Stream* caller = nullptr;
+std::map<const void*, cudaMemoryType> kinds;   // arrays that are not ordinary host memory
 
 void finish(Stream* s) {
   for (const Copy& c : s->queued) std::memcpy(c.dst, c.src, c.n);
@@ -100,8 +101,13 @@ cudaError_t cudaEventSynchronize(cudaEvent_t e) {
   finish(events[e]);
   return cudaSuccess;
 }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
+  a->type = kinds.count(p) ? kinds[p] : cudaMemoryTypeUnregistered;
+  return cudaSuccess;
+}
 cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind, cudaStream_t s) {
   std::lock_guard<std::mutex> g(mu);
+  if (!dst || !src) return cudaErrorInvalidValue;
   if (copies++ == fail_copy) return cudaErrorUnknown;
   of(s)->queued.push_back(Copy{dst, src, n});
   ++(of(s) == caller ? plain : pieces);
@@ -174,6 +180,34 @@ void works() {
   }
 }
 
+// Arrays that are pinned or managed already go by plain copies, the others of
+// the same call by threads.
+void not_pageable(cudaMemoryType t, int n, bool rest_threaded) {
+  for (const bool to_device : {true, false}) {
+    CopyPool pool;
+    fill();
+    kinds.clear();
+    for (int m = 0; m < n; ++m) kinds[host[m].data()] = t;
+    plain = pieces = 0;
+    EXPECT(copy_fields(pool, fields().data(), kFields, kBytes, to_device, stream) == cudaSuccess);
+    cudaStreamSynchronize(stream);
+    EXPECT(plain == (rest_threaded ? n : kFields) && pieces == (rest_threaded ? 2 * (kFields - n) : 0));
+    EXPECT(host == dev);
+  }
+}
+
+// A null pointer is refused with the runtime's error, as by the plain copies.
+void null_pointer() {
+  for (const bool to_device : {true, false}) {
+    CopyPool pool;
+    fill();
+    std::vector<CopyField> f = fields();
+    f[3].host = nullptr;
+    EXPECT(copy_fields(pool, f.data(), kFields, kBytes, to_device, stream) == cudaErrorInvalidValue);
+    cudaStreamSynchronize(stream);
+  }
+}
+
 }  // namespace
 
 int main(int, char** argv) {
@@ -183,6 +217,12 @@ int main(int, char** argv) {
   if (s == "works") works();
   else if (s == "copy_fails") failed(20, -1);
   else if (s == "wait_fails") failed(-1, 5);
+  else if (s == "pinned") not_pageable(cudaMemoryTypeHost, kFields, false);
+  else if (s == "managed") not_pageable(cudaMemoryTypeManaged, kFields, false);
+  else if (s == "some_pinned") not_pageable(cudaMemoryTypeHost, 4, true);
+  else if (s == "few_pageable") not_pageable(cudaMemoryTypeHost, 8, false);   // 5.2 MB of pageable arrays
+  else if (s == "device") not_pageable(cudaMemoryTypeDevice, kFields, false);
+  else if (s == "null") null_pointer();
   else return 2;
   EXPECT(pinned.empty());   // given back with the pool
   return 0;

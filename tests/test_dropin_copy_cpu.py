@@ -26,8 +26,10 @@ def check(tmp_path_factory):
 
 
 # works: the threaded form itself.  copy_fails, wait_fails: one worker's copy
-# or wait fails while the others have pieces in flight
-@pytest.mark.parametrize("scenario", ["works", "copy_fails", "wait_fails"])
+# or wait fails while the others have pieces in flight.  The others: arrays that
+# are not ordinary host memory, all of them or some, and a null pointer
+@pytest.mark.parametrize("scenario", ["works", "copy_fails", "wait_fails", "pinned", "managed", "some_pinned",
+                                      "few_pageable", "device", "null"])
 def test_copies(check, scenario):
     r = subprocess.run([check, scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, (r.returncode, r.stderr)
