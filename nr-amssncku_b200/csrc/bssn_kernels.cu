@@ -142,6 +142,11 @@ Coef<T> make_coef(const double dx[3], double eps) {
     c.h[d] = (T)dx[d];
     c.hinv[d] = T(1) / c.h[d];
   }
+  c.hpow2 = 1;
+  for (int d = 0; d < 3; ++d) {
+    int e;
+    if (!(dx[d] > 0.0) || std::frexp(dx[d], &e) != 0.5) c.hpow2 = 0;
+  }
   c.Fxy = (T)(F1o144 / (dx[0] * dx[1]));
   c.Fxz = (T)(F1o144 / (dx[0] * dx[2]));
   c.Fyz = (T)(F1o144 / (dx[1] * dx[2]));

@@ -264,10 +264,28 @@ __device__ __forceinline__ A lop_term(const FN& f, A b, A bd, int codes) {
   return r;
 }
 
+// a / dx of a KO line sum.  FP64: the product with the rounded reciprocal,
+// corrected by its remainder (Markstein 1990, "Computation of elementary
+// functions on the IBM RISC System/6000 processor"): the rounded quotient in
+// four operations instead of a division (below 1e-305, where the remainder is
+// subnormal, one unit in the last place off); an infinite quotient, whose
+// remainder is no number, stays as it is.
+template <typename T>
+__device__ __forceinline__ T ko_quotient(T a, const Coef<T>& c, int d) {
+  if constexpr (sizeof(T) == 8) {
+    const T q = a * c.hinv[d];
+    const T r = fma(fma(-q, c.h[d], a), c.hinv[d], q);
+    return fabs(q) < T(1.7976931348623157e308) ? r : q;
+  } else {
+    return a * c.hinv[d];
+  }
+}
+
 // KO dissipation of a point from its three lines.
 template <typename A, typename FX, typename FY, typename FZ>
 __device__ __forceinline__ A ko_term(const FX& X, const FY& Y, const FZ& Z, const Coef<A>& C) {
-  return kodiv(ko_sum_rn<A, false>(X), C, 0) + kodiv(ko_sum_rn<A, false>(Y), C, 1) + kodiv(ko_sum_rn<A, false>(Z), C, 2);
+  return ko_quotient(ko_sum_rn<A, false>(X), C, 0) + ko_quotient(ko_sum_rn<A, false>(Y), C, 1) +
+         ko_quotient(ko_sum_rn<A, false>(Z), C, 2);
 }
 
 // March one field of one tile.  A: stencil arithmetic type, S: type of the
