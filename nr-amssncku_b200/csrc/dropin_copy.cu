@@ -10,7 +10,7 @@
 // overlap: 21.4 -> 9.4 ms a call with 16 cores.  The pool belongs to the calling thread's context:
 // kCopyWorkers streams and 2 kCopyWorkers pieces of kCopyPiece bytes, freed
 // with it.  Small calls, calls that get no pool, and arrays that are not ordinary
-// host memory take the plain copies.
+// host memory and outputs that share memory take the plain copies.
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -111,6 +111,17 @@ bool pageable(const void* p) {
   return a.type == cudaMemoryTypeUnregistered;
 }
 
+// Whether two fields share host memory: of outputs that do, the later field's
+// values stay, which only copies one after another keep.
+bool share_memory(const CopyField* fields, int nfields, size_t bytes) {
+  std::vector<const char*> at;
+  for (int m = 0; m < nfields; ++m) at.push_back((const char*)fields[m].host);
+  std::sort(at.begin(), at.end());
+  for (int m = 1; m < nfields; ++m)
+    if ((size_t)(at[m] - at[m - 1]) < bytes) return true;
+  return false;
+}
+
 }  // namespace
 
 cudaError_t copy_fields(CopyPool& P, const CopyField* fields, int nfields, size_t bytes, bool to_device,
@@ -119,7 +130,7 @@ cudaError_t copy_fields(CopyPool& P, const CopyField* fields, int nfields, size_
   // the fields that the threads take
   std::vector<bool> threaded(nfields, false);
   size_t total = 0;
-  if (bytes * nfields >= kLeast)
+  if (bytes * nfields >= kLeast && (to_device || !share_memory(fields, nfields, bytes)))
     for (int m = 0; m < nfields; ++m)
       if (pageable(fields[m].host)) {
         threaded[m] = true;

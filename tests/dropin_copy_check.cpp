@@ -208,6 +208,39 @@ void null_pointer() {
   }
 }
 
+// Output arrays that share memory hold the later field's values, as after
+// copies one after another; inputs that do are only read.
+void shared(size_t offset) {
+  CopyPool pool;
+  fill();
+  std::vector<CopyField> f = fields();
+  host[2].resize(kBytes + offset);
+  f[7].host = host[2].data() + offset;
+  f[2].host = host[2].data();
+  plain = pieces = 0;
+  EXPECT(copy_fields(pool, f.data(), kFields, kBytes, false, stream) == cudaSuccess);
+  cudaStreamSynchronize(stream);
+  EXPECT(plain == kFields && pieces == 0);
+  EXPECT(std::memcmp(f[7].host, dev[7].data(), kBytes) == 0);
+  plain = pieces = 0;
+  EXPECT(copy_fields(pool, f.data(), kFields, kBytes, true, stream) == cudaSuccess);
+  EXPECT(plain == 0 && pieces == 2 * kFields);
+  EXPECT(std::memcmp(f[7].host, dev[7].data(), kBytes) == 0 && std::memcmp(f[2].host, dev[2].data(), kBytes) == 0);
+}
+
+// Outputs that lie one behind the other share nothing.
+void adjacent() {
+  CopyPool pool;
+  fill();
+  std::vector<char> all(kFields * kBytes);
+  std::vector<CopyField> f = fields();
+  for (int m = 0; m < kFields; ++m) f[m].host = all.data() + m * kBytes;
+  plain = pieces = 0;
+  EXPECT(copy_fields(pool, f.data(), kFields, kBytes, false, stream) == cudaSuccess);
+  EXPECT(plain == 0 && pieces == 2 * kFields);
+  for (int m = 0; m < kFields; ++m) EXPECT(std::memcmp(f[m].host, dev[m].data(), kBytes) == 0);
+}
+
 }  // namespace
 
 int main(int, char** argv) {
@@ -223,6 +256,9 @@ int main(int, char** argv) {
   else if (s == "few_pageable") not_pageable(cudaMemoryTypeHost, 8, false);   // 5.2 MB of pageable arrays
   else if (s == "device") not_pageable(cudaMemoryTypeDevice, kFields, false);
   else if (s == "null") null_pointer();
+  else if (s == "same_array") shared(0);
+  else if (s == "overlap") shared(sizeof(double));
+  else if (s == "adjacent") adjacent();
   else return 2;
   EXPECT(pinned.empty());   // given back with the pool
   return 0;
