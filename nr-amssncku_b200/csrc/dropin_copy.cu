@@ -39,9 +39,16 @@ void CopyPool::release() {
 }
 
 bool CopyPool::init() {
-  if (ready || failed) return ready;
-  bool ok = cudaGetDevice(&device) == cudaSuccess &&
-            cudaHostAlloc((void**)&pinned, 2 * kCopyWorkers * kCopyPiece, cudaHostAllocDefault) == cudaSuccess;
+  if (failed) return false;
+  int now = 0;
+  if (cudaGetDevice(&now) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  // the caller has since chosen another device: the runtime's copies serve it
+  if (ready) return now == device;
+  device = now;
+  bool ok = cudaHostAlloc((void**)&pinned, 2 * kCopyWorkers * kCopyPiece, cudaHostAllocDefault) == cudaSuccess;
   for (int w = 0; ok && w < kCopyWorkers; ++w) {
     ok = cudaStreamCreateWithFlags(&stream[w], cudaStreamNonBlocking) == cudaSuccess;
     for (int s = 0; ok && s < 2; ++s) ok = cudaEventCreateWithFlags(&done[w][s], cudaEventDisableTiming) == cudaSuccess;
@@ -71,7 +78,6 @@ void work(CopyPool& P, int w, const std::vector<Piece>& v, std::atomic<size_t>& 
     if (e != cudaSuccess) err.store((int)e);
     return e == cudaSuccess;
   };
-  if (!ck(cudaSetDevice(P.device))) return;
   const Piece* held[2] = {nullptr, nullptr};   // the piece in flight in each slot
   auto settle = [&](int s) {
     if (!held[s]) return true;
@@ -158,7 +164,11 @@ cudaError_t copy_fields(CopyPool& P, const CopyField* fields, int nfields, size_
     t.reserve(nw);
     try {
       for (int w = 1; w < nw; ++w)
-        t.emplace_back([&, w] { work(P, w, v, next, to_device, err); });
+        t.emplace_back([&, w] {
+          const cudaError_t d = cudaSetDevice(P.device);   // a thread starts on device 0
+          if (d != cudaSuccess) err.store((int)d);
+          else work(P, w, v, next, to_device, err);
+        });
     } catch (const std::exception&) {   // no more threads, or no memory for one: those there are, and this one, do it
     }
     work(P, 0, v, next, to_device, err);

@@ -17,7 +17,7 @@ struct CopyPool {
   int device = 0;
   bool ready = false, failed = false;
   ~CopyPool();
-  bool init();
+  bool init();   // whether there are pieces on the calling thread's device
   void release();
   char* slot(int w, int s) { return pinned + (size_t)(2 * w + s) * kCopyPiece; }
 };

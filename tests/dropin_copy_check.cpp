@@ -33,12 +33,14 @@ int copies = 0, waits = 0;                 // calls so far
 int fail_copy = -1, fail_wait = -1;        // the call that fails, counted from 0
 int plain = 0, pieces = 0;                 // copies on the caller's stream, and on others
 Stream* caller = nullptr;
+thread_local int device = 0;               // each thread's current device
 std::map<const void*, cudaMemoryType> kinds;   // arrays that are not ordinary host memory
 
 void finish(Stream* s) {
   for (const Copy& c : s->queued) std::memcpy(c.dst, c.src, c.n);
   s->queued.clear();
 }
+bool wrong_device = false;                 // a worker's copy issued on another device than the pool's (1)
 size_t in_flight() {
   size_t n = 0;
   for (Stream* s : streams) n += s->queued.size();
@@ -49,8 +51,8 @@ Stream* of(cudaStream_t s) { return reinterpret_cast<Stream*>(s); }
 }  // namespace
 
 extern "C" {
-cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
-cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetDevice(int* d) { *d = device; return cudaSuccess; }
+cudaError_t cudaSetDevice(int d) { device = d; return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
   std::lock_guard<std::mutex> g(mu);
@@ -106,6 +108,7 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
   return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind, cudaStream_t s) {
+  if (of(s) != caller && device != 1) wrong_device = true;
   std::lock_guard<std::mutex> g(mu);
   if (!dst || !src) return cudaErrorInvalidValue;
   if (copies++ == fail_copy) return cudaErrorUnknown;
@@ -241,6 +244,25 @@ void adjacent() {
   for (int m = 0; m < kFields; ++m) EXPECT(std::memcmp(f[m].host, dev[m].data(), kBytes) == 0);
 }
 
+// The copies leave the calling thread's current device as it is, and a call
+// made on another device than the pool's takes the plain copies.
+void devices() {
+  CopyPool pool;
+  cudaSetDevice(1);
+  fill();
+  wrong_device = false;
+  EXPECT(copy_fields(pool, fields().data(), kFields, kBytes, true, stream) == cudaSuccess);
+  EXPECT(device == 1 && !wrong_device && host == dev);
+  cudaSetDevice(2);
+  for (const bool to_device : {true, false}) {
+    fill();
+    plain = pieces = 0;
+    EXPECT(copy_fields(pool, fields().data(), kFields, kBytes, to_device, stream) == cudaSuccess);
+    cudaStreamSynchronize(stream);
+    EXPECT(device == 2 && plain == kFields && pieces == 0 && host == dev);
+  }
+}
+
 }  // namespace
 
 int main(int, char** argv) {
@@ -259,6 +281,7 @@ int main(int, char** argv) {
   else if (s == "same_array") shared(0);
   else if (s == "overlap") shared(sizeof(double));
   else if (s == "adjacent") adjacent();
+  else if (s == "devices") devices();
   else return 2;
   EXPECT(pinned.empty());   // given back with the pool
   return 0;
