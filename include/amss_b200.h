@@ -284,10 +284,13 @@ int amss_engine_run_graph(amss_engine* e, int level, double dt, int nsteps, int 
  * default, the block's x extent cut into equal pieces of at most 38) and the
  * number of z-slabs each block's march is cut into (1..16; slabs are at least
  * 8 planes).  0 and 1 together, the initial setting, let the engine choose the
- * slabs.  Results do not depend on it.  Waits for the engine's stream; not
- * inside a stream capture. */
+ * slabs (of at least 4 planes); one slab at the default width is 38 and 1.
+ * Results do not depend on it.  Waits for the engine's stream; not inside a
+ * stream capture. */
 int amss_engine_set_level_tiling(amss_engine* e, int level, int tile_w, int zsplit);
-/* The level's tiling (as set; 0 = default width) and its stencil work items. */
+/* The level's tiling as set (0 = default width; 0 and 1: the engine's own slabs,
+ * however many it uses) and its stencil work items, from which the slabs in use
+ * follow. */
 int amss_engine_get_level_tiling(amss_engine* e, int level, int* tile_w, int* zsplit, int* nitems);
 /* No reference counterpart: a level's occupancy setting, 0 (the default) or 1.
  * The stencil pass has one compiled form, two resident CTAs per SM, so the

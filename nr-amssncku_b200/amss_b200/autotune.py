@@ -19,29 +19,31 @@ import numpy as np
 
 from .engine import Engine
 
+WIDEST = 38   # columns of the stencil pass's widest tile
 DEFAULT_CACHE = os.path.join(os.path.expanduser("~"), ".cache", "amss_b200", "tiling.json")
 
 
 def level_key(H, level, precision, formulation):
     shapes = sorted(tuple(H.blocks[i].ex) for p in H.levels[level] for i in p.blocks)
-    # tile38: the stencil pass's widest tile; times of passes with other tiles don't carry over
-    return f"{precision}/{formulation}/tile38/" + ";".join("x".join(map(str, s)) for s in shapes)
+    # times of passes with other widest tiles don't carry over
+    return f"{precision}/{formulation}/tile{WIDEST}/" + ";".join("x".join(map(str, s)) for s in shapes)
 
 
 def candidates(H, level):
-    """(tile width, z-split, occupancy) worth timing for a level: the default
-    width and the widths that cut the level's smallest block width into 1-3
-    near-equal tiles, each with 1-4 z-slabs (occupancy 0: one compiled form)."""
+    """(tile width, z-split, occupancy setting) worth timing for a level: the
+    default width and the widths that cut the level's smallest block width into
+    1-3 near-equal tiles, each with 1-4 z-slabs.  (0, 1) is the engine's own
+    choice of slabs; the default width in one slab is (38, 1), the widest tile."""
     wmin = min(H.blocks[i].ex[0] for p in H.levels[level] for i in p.blocks)
     widths = {0}
     for parts in (1, 2, 3):
         w = -(-wmin // parts)
-        if 8 <= w <= 38:
+        if 8 <= w <= WIDEST:
             widths.add(w)
     for w in (16, 32):
         if w <= wmin:
             widths.add(w)
-    return [(w, z, o) for w in sorted(widths) for z in (1, 2, 3, 4) for o in (0,)]
+    return [(w, z, 0) for w in sorted(widths) for z in (1, 2, 3, 4)] + [(WIDEST, 1, 0)] * (WIDEST not in widths)
 
 
 def _time_level(eng, level, dt, reps):

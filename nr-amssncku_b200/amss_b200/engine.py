@@ -178,7 +178,8 @@ class Engine:
     def set_level_tiling(self, level, tile_w=0, zsplit=1):
         """Stencil-pass tiling of one level (amss_engine_set_level_tiling):
         tile width 8..64, at most 38 used (0: default), and z-slabs per
-        block; (0, 1) lets the engine choose the slabs."""
+        block; (0, 1) lets the engine choose the slabs, (38, 1) is one slab
+        at the default width."""
         check(lib().amss_engine_set_level_tiling(self._h, level, int(tile_w), int(zsplit)),
               "amss_engine_set_level_tiling")
 

@@ -1,7 +1,8 @@
-"""The stencil pass's per-level tiling and occupancy form
-(amss_engine_set_level_tiling, amss_engine_set_level_occupancy) and their
-autotuner (amss_b200.autotune): every tiling and form computes the same
-numbers, bit for bit, and the tuner returns a valid choice for every level."""
+"""The stencil pass's per-level tiling (amss_engine_set_level_tiling) and its
+autotuner (amss_b200.autotune): every tiling computes the same numbers, bit for
+bit, and the tuner returns a valid choice for every level.  The occupancy setting
+(amss_engine_set_level_occupancy) is recorded and returned; no kernel depends on
+it."""
 import numpy as np
 import pytest
 
