@@ -287,7 +287,10 @@ extern "C" amss_adjoint* amss_adjoint_create(const int ex[3], const double bbox[
                                 F_AXY, F_AXZ, F_AYY, F_AYZ, F_AZZ, F_DTSFX, F_DTSFY, F_DTSFZ};
   const int lo[3] = {0, 0, 0};
   deriv_push(cut, 0, lo, ex, DWMAX, 1, kAutoSlab);
-  const int slabs = deriv_slabs(cut, false, 2 * 148);
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int slabs = deriv_slabs(cut, false, 2 * sms);
   cut.clear();
   deriv_push(cut, 0, lo, ex, DWMAX, slabs, kAutoSlab);
   // the transpose's tiles, and its slabs by the same rule (its warm-up and
@@ -296,7 +299,7 @@ extern "C" amss_adjoint* amss_adjoint_create(const int ex[3], const double bbox[
   const int tw = tg_tile_w(ex[0]), th = DTHREADS / tw;
   for (int y0 = 0; y0 < ex[1]; y0 += th)
     for (int x0 = 0; x0 < ex[0]; x0 += tw) gcut.push_back(DerivItem{0, x0, y0, 0, 0, ex[2], ex[0], ex[1], tw, th});
-  const int gslabs = std::min(deriv_slabs(gcut, false, 2 * 148), ex[2] / kAutoSlab);
+  const int gslabs = std::min(deriv_slabs(gcut, false, 2 * sms), ex[2] / kAutoSlab);
   for (int f : order) {
     for (DerivItem it : cut) {
       it.field = f;

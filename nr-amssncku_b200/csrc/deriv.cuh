@@ -582,11 +582,8 @@ __device__ __forceinline__ void deriv_march(const StepBlock<T>& B, const S* src,
 
 // Stencil pass over a work list of (block, tile, slab, field) items, ordered
 // by field so that resident CTAs share one code path.
-#ifndef AMSS_DMINB
-#define AMSS_DMINB 2
-#endif
 template <typename T, typename SI, bool Z4C>
-__global__ void __launch_bounds__(DTHREADS, AMSS_DMINB) k_deriv(const StepBlock<T>* __restrict__ blocks,
+__global__ void __launch_bounds__(DTHREADS, 2) k_deriv(const StepBlock<T>* __restrict__ blocks,
                                                        const DerivItem* __restrict__ items, int nitems, int sub,
                                                        T* __restrict__ D, int slots, int region, int spare) {
   extern __shared__ __align__(16) unsigned char smem[];

@@ -9,7 +9,7 @@
 // 70^3 points, 28 % of DRAM bandwidth).  Each warp therefore copies the rows
 // of its 32 points into a shared-memory region of its own, with cp.async and
 // several groups ahead of their use (25 KB a warp, 200 KB of an SM), and the
-// point function reads shared memory: 165 us on 70^3 points, 4.2 TB/s; Z4c on
+// point function reads shared memory: 160-173 us on 70^3 points, 3.4-3.9 TB/s; Z4c on
 // 134^3 points 2,103 -> 1,110 us; the mixed form on 70^3 points 205 -> 120 us.
 // No CTA barrier: a warp waits for its own copies only.  What remains is the
 // latency of dependent FP64 operations at two warps a scheduler.
@@ -109,12 +109,6 @@ struct PwStage {
 __device__ __forceinline__ void cp_async16(unsigned sdst, const void* gsrc) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sdst), "l"(gsrc) : "memory");
 }
-__device__ __forceinline__ void cp_async8_at(unsigned sdst, const void* gsrc) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sdst), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async4_at(unsigned sdst, const void* gsrc) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sdst), "l"(gsrc) : "memory");
-}
 
 // Accessor of the pointwise pass over a warp's staged rows.
 template <typename T, typename SI, bool Z4C>
@@ -139,9 +133,9 @@ struct StagedPt {
       if constexpr (S::kCentre) {
 #pragma unroll
         for (int F = 0; F < S::kNf; ++F) {
-          if constexpr (sizeof(SI) == 8) cp_async8_at(sreg + S::off_c(F) + lane * 8, in + F * fs);
-          else if (is_wide(F)) cp_async8_at(sreg + S::off_c(F) + lane * 8, in_side + side_slot(F) * fs);
-          else cp_async4_at(sreg + S::off_c(F) + lane * 4, in + F * fs);
+          if constexpr (sizeof(SI) == 8) cp_async8(sreg + S::off_c(F) + lane * 8, in + F * fs);
+          else if (is_wide(F)) cp_async8(sreg + S::off_c(F) + lane * 8, in_side + side_slot(F) * fs);
+          else cp_async4(sreg + S::off_c(F) + lane * 4, in + F * fs);
         }
       }
     } else {
@@ -150,13 +144,13 @@ struct StagedPt {
 #pragma unroll
       for (int i = 0; i < S::nput(PH); ++i) {
         const int F = S::put_field(PH, i);
-        cp_async8_at(sreg + S::start(PH) + (S::nd(PH) + S::ndz(PH)) * S::kRow + i * S::kRow8 + lane * 8, u0 + F * fs);
+        cp_async8(sreg + S::start(PH) + (S::nd(PH) + S::ndz(PH)) * S::kRow + i * S::kRow8 + lane * 8, u0 + F * fs);
       }
       if (S::nput(PH) > 0 && sub != 0) {
 #pragma unroll
         for (int i = 0; i < S::nput(PH); ++i) {
           const int F = S::put_field(PH, i);
-          cp_async8_at(sreg + S::start(PH) + (S::nd(PH) + S::ndz(PH)) * S::kRow + (S::nput(PH) + i) * S::kRow8 + lane * 8,
+          cp_async8(sreg + S::start(PH) + (S::nd(PH) + S::ndz(PH)) * S::kRow + (S::nput(PH) + i) * S::kRow8 + lane * 8,
                        K + F * fs);
         }
       }
