@@ -247,7 +247,7 @@ extern "C" int compute_rhs_bssn_(
   int nio = 0;
   for (int f = 0; f < 24; ++f) io[nio++] = {du + f * fs, st_in[f]};
   for (int f = 0; f < 10; ++f) io[nio++] = {dm + f * fs, mat[f]};
-  AMSS_CK(copy_fields(c.pool, io, nio, bytes, true, s));
+  AMSS_CK(copy_fields(copy_pools(), io, nio, bytes, true, s));
   AMSS_CK(cudaMemcpyAsync(dX, X, ex[0] * sizeof(double), cudaMemcpyHostToDevice, s));
   AMSS_CK(cudaMemcpyAsync(dY, Y, ex[1] * sizeof(double), cudaMemcpyHostToDevice, s));
   AMSS_CK(cudaMemcpyAsync(dZ, Z, ex[2] * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -280,7 +280,7 @@ extern "C" int compute_rhs_bssn_(
   for (int f = 0; f < 6; ++f) io[nio++] = {dR + f * fs, rc[f]};
   if (*co == 0)
     for (int f = 0; f < 7; ++f) io[nio++] = {dc + f * fs, cs[f]};
-  AMSS_CK(copy_fields(c.pool, io, nio, bytes, false, s));
+  AMSS_CK(copy_fields(copy_pools(), io, nio, bytes, false, s));
   AMSS_CK(cudaStreamSynchronize(s));
   return 0;
 }
@@ -338,7 +338,7 @@ extern "C" int compute_rhs_z4c_(
   int nio = 0;
   for (int f = 0; f < 25; ++f) io[nio++] = {du + f * fs, st_in[f]};
   for (int f = 0; f < 10; ++f) io[nio++] = {dm + f * fs, mat[f]};
-  AMSS_CK(copy_fields(c.pool, io, nio, bytes, true, s));
+  AMSS_CK(copy_fields(copy_pools(), io, nio, bytes, true, s));
   AMSS_CK(cudaMemcpyAsync(dX, X, ex[0] * sizeof(double), cudaMemcpyHostToDevice, s));
   AMSS_CK(cudaMemcpyAsync(dY, Y, ex[1] * sizeof(double), cudaMemcpyHostToDevice, s));
   AMSS_CK(cudaMemcpyAsync(dZ, Z, ex[2] * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -375,7 +375,7 @@ extern "C" int compute_rhs_z4c_(
   for (int f = 0; f < 18; ++f) io[nio++] = {dg + f * fs, gm[f]};
   for (int f = 0; f < 6; ++f) io[nio++] = {dR + f * fs, rc[f]};
   for (int f = 0; f < 7; ++f) io[nio++] = {dc + f * fs, cs[f]};
-  AMSS_CK(copy_fields(c.pool, io, nio, bytes, false, s));
+  AMSS_CK(copy_fields(copy_pools(), io, nio, bytes, false, s));
   AMSS_CK(cudaStreamSynchronize(s));
   return 0;
 }

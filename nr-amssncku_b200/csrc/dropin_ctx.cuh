@@ -2,12 +2,15 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <memory>
+#include <mutex>
+#include <vector>
+
 #include "dev_util.cuh"
 
 namespace amss {
 
-// Pinned pieces and streams of the threaded copies (dropin_copy.cu), made at
-// the first large copy.
+// Pinned pieces and streams of the threaded copies (dropin_copy.cu).
 constexpr int kCopyWorkers = 8;
 constexpr size_t kCopyPiece = (size_t)1 << 20;
 struct CopyPool {
@@ -15,19 +18,34 @@ struct CopyPool {
   cudaStream_t stream[kCopyWorkers] = {};
   cudaEvent_t done[kCopyWorkers][2] = {};
   int device = 0;
-  bool ready = false, failed = false;
   ~CopyPool();
-  bool init();   // whether there are pieces on the calling thread's device
-  void release();
+  bool init(int dev);
   char* slot(int w, int s) { return pinned + (size_t)(2 * w + s) * kCopyPiece; }
 };
+// The process's pools: a call takes one and gives it back, so that threads that
+// call one after another share it.  A pool costs 9 to 20 ms to make (16 MB of
+// pinned memory) and saves about 40 us a MB, so it is made once kPoolEarned
+// bytes have been copied without it; at most kMaxPools, kept to the end of the
+// process.
+constexpr int kMaxPools = 4;
+constexpr size_t kPoolEarned = (size_t)256 << 20;
+struct CopyPools {
+  std::mutex lock;
+  std::vector<std::unique_ptr<CopyPool>> idle;
+  int made = 0;
+  size_t plain = 0;      // bytes copied for want of a pool since the last was made
+  bool failed = false;   // a pool could not be made, or a copy through one failed: no more of them
+  std::unique_ptr<CopyPool> take(size_t bytes);   // on the calling thread's device; null: plain copies
+  void give(std::unique_ptr<CopyPool> pool);
+};
+CopyPools& copy_pools();
 struct CopyField {
   void* dev;
   void* host;
 };
 // Copies `bytes` of every field host -> device or back.  In stream order with
 // s; the copies that threads made have also completed on return.
-cudaError_t copy_fields(CopyPool& pool, const CopyField* fields, int nfields, size_t bytes, bool to_device,
+cudaError_t copy_fields(CopyPools& pools, const CopyField* fields, int nfields, size_t bytes, bool to_device,
                         cudaStream_t s);
 
 // Per-thread device scratch of the drop-in entries (grow-only, reused).
@@ -36,7 +54,6 @@ struct DropinCtx {
   double* dbuf = nullptr;
   size_t cap = 0;      // doubles
   unsigned* dstatus = nullptr;
-  CopyPool pool;
   bool ok = false;
   ~DropinCtx() {
     if (dbuf) cudaFree(dbuf);

@@ -11,6 +11,7 @@
 #include <mutex>
 #include <set>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "dropin_ctx.cuh"
@@ -29,6 +30,7 @@ std::mutex mu;
 std::set<Stream*> streams;
 std::map<void*, Stream*> events;           // event -> stream it was recorded on
 std::vector<char*> pinned;                 // live pinned buffers
+int allocations = 0;                       // pinned buffers made so far
 int copies = 0, waits = 0;                 // calls so far
 int fail_copy = -1, fail_wait = -1;        // the call that fails, counted from 0
 int plain = 0, pieces = 0;                 // copies on the caller's stream, and on others
@@ -57,6 +59,7 @@ cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
   std::lock_guard<std::mutex> g(mu);
   pinned.push_back((char*)(*p = std::malloc(n)));
+  ++allocations;
   return cudaSuccess;
 }
 cudaError_t cudaFreeHost(void* p) {
@@ -108,8 +111,8 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
   return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind, cudaStream_t s) {
-  if (of(s) != caller && device != 1) wrong_device = true;
   std::lock_guard<std::mutex> g(mu);
+  if (of(s) != caller && device != 1) wrong_device = true;
   if (!dst || !src) return cudaErrorInvalidValue;
   if (copies++ == fail_copy) return cudaErrorUnknown;
   of(s)->queued.push_back(Copy{dst, src, n});
@@ -135,6 +138,11 @@ constexpr size_t kBytes = (size_t)1300 * 1000;   // a piece and a remainder; 15.
 std::vector<std::vector<char>> host(kFields), dev(kFields);
 cudaStream_t stream;
 
+// Pools of which the next large call makes one.
+struct Ready : CopyPools {
+  Ready() { plain = kPoolEarned; }
+};
+
 std::vector<CopyField> fields() {
   std::vector<CopyField> f;
   for (int m = 0; m < kFields; ++m) f.push_back(CopyField{dev[m].data(), host[m].data()});
@@ -155,7 +163,7 @@ void fill() {
 // arrays may be reused at once.  The calls after it take the plain copies.
 void failed(int at_copy, int at_wait) {
   for (const bool to_device : {true, false}) {
-    CopyPool pool;
+    Ready pool;
     fill();
     copies = waits = 0;
     fail_copy = at_copy;
@@ -174,7 +182,7 @@ void failed(int at_copy, int at_wait) {
 
 void works() {
   for (const bool to_device : {true, false}) {
-    CopyPool pool;
+    Ready pool;
     fill();
     plain = pieces = 0;
     EXPECT(copy_fields(pool, fields().data(), kFields, kBytes, to_device, stream) == cudaSuccess);
@@ -187,7 +195,7 @@ void works() {
 // the same call by threads.
 void not_pageable(cudaMemoryType t, int n, bool rest_threaded) {
   for (const bool to_device : {true, false}) {
-    CopyPool pool;
+    Ready pool;
     fill();
     kinds.clear();
     for (int m = 0; m < n; ++m) kinds[host[m].data()] = t;
@@ -202,7 +210,7 @@ void not_pageable(cudaMemoryType t, int n, bool rest_threaded) {
 // A null pointer is refused with the runtime's error, as by the plain copies.
 void null_pointer() {
   for (const bool to_device : {true, false}) {
-    CopyPool pool;
+    Ready pool;
     fill();
     std::vector<CopyField> f = fields();
     f[3].host = nullptr;
@@ -214,7 +222,7 @@ void null_pointer() {
 // Output arrays that share memory hold the later field's values, as after
 // copies one after another; inputs that do are only read.
 void shared(size_t offset) {
-  CopyPool pool;
+  Ready pool;
   fill();
   std::vector<CopyField> f = fields();
   host[2].resize(kBytes + offset);
@@ -233,7 +241,7 @@ void shared(size_t offset) {
 
 // Outputs that lie one behind the other share nothing.
 void adjacent() {
-  CopyPool pool;
+  Ready pool;
   fill();
   std::vector<char> all(kFields * kBytes);
   std::vector<CopyField> f = fields();
@@ -247,7 +255,7 @@ void adjacent() {
 // The copies leave the calling thread's current device as it is, and a call
 // made on another device than the pool's takes the plain copies.
 void devices() {
-  CopyPool pool;
+  Ready pool;
   cudaSetDevice(1);
   fill();
   wrong_device = false;
@@ -261,6 +269,48 @@ void devices() {
     cudaStreamSynchronize(stream);
     EXPECT(device == 2 && plain == kFields && pieces == 0 && host == dev);
   }
+}
+
+// Calls that each come from a thread of their own share a pool, and none is
+// made before its cost is earned.
+void thread_a_call() {
+  CopyPools pools;
+  const size_t all = kFields * kBytes;
+  size_t done = 0;
+  for (int call = 0; call < 60; ++call, done += all) {
+    fill();
+    plain = pieces = 0;
+    cudaError_t e = cudaErrorUnknown;
+    std::thread([&] { e = copy_fields(pools, fields().data(), kFields, kBytes, call & 1, stream); }).join();
+    EXPECT(e == cudaSuccess);
+    cudaStreamSynchronize(stream);
+    EXPECT(host == dev);
+    EXPECT(done < kPoolEarned ? plain == kFields && allocations == 0 : pieces == 2 * kFields && allocations == 1);
+  }
+}
+
+// Six threads at once: at most kMaxPools pools, and each thread's own data.
+void threads_at_once() {
+  CopyPools pools;
+  std::vector<std::thread> t;
+  std::vector<int> good(6, 0);
+  for (int k = 0; k < 6; ++k)
+    t.emplace_back([&, k] {
+      const size_t bytes = 3 << 20;
+      std::vector<std::vector<char>> h(4, std::vector<char>(bytes)), d(4, std::vector<char>(bytes));
+      std::vector<CopyField> f;
+      for (int m = 0; m < 4; ++m) f.push_back(CopyField{d[m].data(), h[m].data()});
+      for (int call = 0; call < 40; ++call) {
+        for (int m = 0; m < 4; ++m) std::memset((call & 1 ? h : d)[m].data(), 31 * k + 7 * m + call, bytes);
+        if (copy_fields(pools, f.data(), 4, bytes, call & 1, stream) != cudaSuccess) return;
+        cudaStreamSynchronize(stream);
+        if (h != d) return;
+      }
+      good[k] = 1;
+    });
+  for (auto& x : t) x.join();
+  EXPECT(std::count(good.begin(), good.end(), 1) == 6);
+  EXPECT(allocations >= 1 && allocations <= kMaxPools);
 }
 
 }  // namespace
@@ -282,6 +332,8 @@ int main(int, char** argv) {
   else if (s == "overlap") shared(sizeof(double));
   else if (s == "adjacent") adjacent();
   else if (s == "devices") devices();
+  else if (s == "thread_a_call") thread_a_call();
+  else if (s == "threads_at_once") threads_at_once();
   else return 2;
   EXPECT(pinned.empty());   // given back with the pool
   return 0;

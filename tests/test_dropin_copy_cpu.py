@@ -28,10 +28,11 @@ def check(tmp_path_factory):
 # works: the threaded form itself.  copy_fails, wait_fails: one worker's copy
 # or wait fails while the others have pieces in flight.  The others: arrays that
 # are not ordinary host memory, all of them or some, a null pointer, and output
-# arrays that share memory or just do not; and a caller that changes its device
+# arrays that share memory or just do not; a caller that changes its device; and
+# calls from many threads, one after another and at once
 @pytest.mark.parametrize("scenario", ["works", "copy_fails", "wait_fails", "pinned", "managed", "some_pinned",
                                       "few_pageable", "device", "null", "same_array", "overlap", "adjacent",
-                                      "devices"])
+                                      "devices", "thread_a_call", "threads_at_once"])
 def test_copies(check, scenario):
     r = subprocess.run([check, scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, (r.returncode, r.stderr)

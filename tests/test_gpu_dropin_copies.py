@@ -1,6 +1,6 @@
 """The drop-in right-hand side on arrays large enough for the threaded copies
 (8 MB in all; fields of more than one 1 MB piece, with a remainder): against
-the oracle, and from two threads at once, each with its own pool of pieces."""
+the oracle, and from two threads at once, each with a pool of pieces."""
 import threading
 
 import numpy as np
@@ -17,6 +17,23 @@ pytestmark = pytest.mark.gpu
 def _inputs(ex, seed):
     X = [-2.0 + (np.arange(n) + 0.5) * 0.1 for n in ex]
     return X, generic_state(*X, seed=seed, amp=0.5)
+
+
+@pytest.fixture(scope="module", autouse=True)
+def pools():
+    """A pool is made once 256 MB have been copied for want of one: two threads
+    copy 104 MB a call until there are two."""
+    X, st = _inputs((54, 53, 51), 3)
+
+    def go():
+        for _ in range(8):
+            dropin.compute_rhs_bssn(*X, st, eps=0.1, co=0)
+
+    threads = [threading.Thread(target=go) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
 
 
 def test_smallest_threaded_call_equals_the_plain_copies():
