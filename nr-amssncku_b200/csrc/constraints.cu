@@ -23,11 +23,11 @@ struct EpiNone {   // the right-hand side itself is not wanted
 
 constexpr int kConsThreads = 128;
 
-// residuals of every point of the level into cons (7 fields, the D layout:
-// block offset doff, field stride dfs).  A CTA a tile: the pass waits on the
+// residuals of every point of the level into cons (7 fields: block offset doff,
+// field stride dfs).  A CTA a tile: the pass waits on the
 // loads of its stencils at eight warps an SM (255 registers), and a grid of
 // eight CTAs an SM that loops over the tiles leaves a slot empty while a CTA's
-// last warp finishes: 1,037 us for the norms of 102^3 points, 799 us now.
+// last warp finishes: 1,037 us for the norms of 102^3 points, 808 us now.
 // (168 registers and three CTAs: 883 us, four: 858 us, for their spills.)
 template <typename T, bool SYMM>
 __global__ void __launch_bounds__(kConsThreads) k_constraints(const StepBlock<T>* __restrict__ blocks,

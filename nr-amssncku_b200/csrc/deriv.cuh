@@ -120,7 +120,7 @@ inline void deriv_push(std::vector<DerivItem>& v, int block, const int lo[3], co
 // longest item, or all items shared out plus part of a last one.  A 24^3 block
 // is 48 items of 30 steps uncut and 288 of 10 in six slabs (a step 459 and
 // 216 us); 70^3 points go in two (1.92 ms a step; 2.17 uncut, 1.94 in three,
-// 1.89 in four), 134^3 of Z4c in one or two alike (12.2 and 12.3 ms).
+// 1.90 in four), 134^3 of Z4c in one or two alike (12.4 ms).
 inline int deriv_slabs(const std::vector<DerivItem>& one, bool z4c, int ctas) {
   const double per_tile = 11.0 + (z4c ? 5 : 4) * 0.65 + 9 * 0.5;
   int best = 1;
